@@ -232,6 +232,14 @@ void launch_face_nodes(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face
   }
 }
 
+// The step kernels launch_aa uses (an odd step is always one launch, an even
+// step of two substances always two); the others are not compiled.
+template <int NS, int PART, bool ODD>
+constexpr bool step_part_used()
+{
+  return ODD ? PART == PART_ALL : (NS == 1 || PART != PART_ALL);
+}
+
 template <typename T, int Q, int NS, int MODEL, int PART>
 void launch_part(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fused<T>* f3)
 {
@@ -245,8 +253,9 @@ void launch_part(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fused
     if (C.m_end <= C.m_base) return;
     const bool idx32 = (unsigned long long)Q * (unsigned long long)d->P < (1ull << 32);
     auto go = [&](auto odd_c, auto idx_c, auto oop_c) {
-      aa_step_compact<T, Q, NS, MODEL, decltype(odd_c)::value, PART, decltype(idx_c)::value,
-                      decltype(oop_c)::value><<<blocks, 256, 0, d->stream>>>(C);
+      if constexpr (step_part_used<NS, PART, decltype(odd_c)::value>())
+        aa_step_compact<T, Q, NS, MODEL, decltype(odd_c)::value, PART, decltype(idx_c)::value,
+                        decltype(oop_c)::value><<<blocks, 256, 0, d->stream>>>(C);
     };
     using TT = std::true_type;
     using FF = std::false_type;
@@ -260,23 +269,30 @@ void launch_part(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fused
     d->launches++;
     return;
   }
-  dim3 block(128, 1, 1);
-  dim3 grid((A.LX + 127) / 128, A.LY, A.LZ);
+  const unsigned blocks = (unsigned)((A.N + 255) / 256);
+  const FastDiv dp = make_fastdiv((unsigned)(A.LX * A.LY)), dl = make_fastdiv((unsigned)A.LX);
+  const bool idx32 = (unsigned long long)Q * (unsigned long long)A.N < (1ull << 32);
+  auto go = [&](auto odd_c, auto idx_c, auto walsh_c) {
+    if constexpr (step_part_used<NS, PART, decltype(odd_c)::value>())
+      aa_step<T, Q, NS, MODEL, decltype(odd_c)::value, PART, decltype(idx_c)::value,
+              decltype(walsh_c)::value><<<blocks, 256, 0, d->stream>>>(A, dp, dl);
+  };
+  using TT = std::true_type;
+  using FF = std::false_type;
   if (A.ns) {
-    if (odd) aa_step<T, Q, NS, MODEL, true, PART, true><<<grid, block, 0, d->stream>>>(A);
-    else aa_step<T, Q, NS, MODEL, false, PART, true><<<grid, block, 0, d->stream>>>(A);
+    if (idx32) { if (odd) go(TT{}, TT{}, TT{}); else go(FF{}, TT{}, TT{}); }
+    else { if (odd) go(TT{}, FF{}, TT{}); else go(FF{}, FF{}, TT{}); }
   } else {
-    if (odd) aa_step<T, Q, NS, MODEL, true, PART><<<grid, block, 0, d->stream>>>(A);
-    else aa_step<T, Q, NS, MODEL, false, PART><<<grid, block, 0, d->stream>>>(A);
+    if (idx32) { if (odd) go(TT{}, TT{}, FF{}); else go(FF{}, TT{}, FF{}); }
+    else { if (odd) go(TT{}, FF{}, FF{}); else go(FF{}, FF{}, FF{}); }
   }
   d->launches++;
 }
 
 // One step: a single launch for the flow alone; for two substances, an odd
-// step of the compact layout is one launch too (per node the flow, then the
-// solute from the slots the flow's pulls found, its u in registers; written
-// out of place, for the adjoint's recomputation, it also stores u), and an
-// even step is a flow launch that hands u to a solute launch (the solute
+// step is one launch too (per node the flow, then the solute from the slots
+// the flow's pulls found, its u in registers; written out of place, for the
+// adjoint's recomputation, it also stores u), and an even step is a flow launch that hands u to a solute launch (the solute
 // launch only while the solute is active; fused, the even step spilled and
 // ran slower).
 // With the z faces fused, the face planes' nodes run in a launch of their
@@ -298,7 +314,7 @@ bool launch_aa(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fused<T
   }
   if constexpr (NS == 1) {
     launch_part<T, Q, NS, MODEL, PART_ALL>(d, A, odd, f3);
-  } else if (odd && d->layout == LBX_LAYOUT_COMPACT) {
+  } else if (odd) {
     launch_part<T, Q, NS, MODEL, PART_ALL>(d, A, odd, f3);
   } else {
     launch_part<T, Q, NS, MODEL, PART_FLOW>(d, A, odd, f3);

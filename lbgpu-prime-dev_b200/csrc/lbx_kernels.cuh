@@ -462,37 +462,53 @@ __device__ __forceinline__ void face_south(int kind, T rho_bc, T rhoA, T drho, b
 // WALSH (partial bounce-back, COMPUTE_ON_SOLIDS): every node is updated and
 // streams periodically with no solid checks (src/lattice.c:2704-2707,
 // :2812-2815); the collision blends by ns (see collide).
-template <typename T, int Q, int NS, int MODEL, bool ODD, int PART, bool WALSH = false>
-__global__ void __launch_bounds__(128)
-aa_step(StepArgs<T> A)
+
+// A population load that goes past L1: no thread reads another's slots in
+// the same step, so L1 has nothing to give, and a plain load of a line that
+// neighbouring warps store to holds the store up.
+template <typename T>
+__device__ __forceinline__ T ld_pop(const T* p) { return __ldcg(p); }
+
+// Resident 256-thread blocks of the dense kernels: FP32 six (40 registers),
+// FP64 three (80; two substances' solute two, four for D2Q9's 64); the odd
+// step of two substances in one launch as in the compact layout; Walsh
+// kernels hold the incoming populations too.  Measured at 193 x 161 x 120:
+// FP32 odd 105 us at six or five, 109 at four or seven; even 94 us at six,
+// 101 at four; FP64 odd 185 us at three, 221 at two.
+template <typename T, int Q, int NS, int PART, bool WALSH>
+constexpr int dense_min_blocks()
 {
+  return (PART == PART_ALL && NS == 2) ? (sizeof(T) == 4 && !WALSH ? 4 : 2)
+       : sizeof(T) == 4                ? (WALSH ? 4 : 6)
+       : WALSH                         ? 2
+                                       : (Q == 9 ? 4 : (PART == PART_SOLUTE ? 2 : 3));
+}
+
+// One thread per node, the nodes numbered through (no block starts anew at
+// a row): every warp is full and starts on a 128-byte boundary of its
+// direction planes whatever LX is.  With a block row per lattice row,
+// LX = 193 left a quarter of the lanes idle and every other row misaligned
+// (even step of 193 x 161 x 120 FP32: 104 -> 94 us, 6.05 TB/s).
+// The odd step keeps its pull slots in shared memory, one column per
+// thread, as the compact kernel does: the push writes d_a to the slot
+// d_opp(a) was pulled from, so no address is formed twice (its registers
+// and 64-bit address arithmetic bound the step: 140 -> 105 us FP32,
+// 231 -> 185 us FP64).  IDX32: offsets within one substance's [Q][N] block
+// fit in 32 bits.
+template <typename T, int Q, int NS, int MODEL, bool ODD, int PART, bool IDX32, bool WALSH = false>
+__global__ void __launch_bounds__(256, (dense_min_blocks<T, Q, NS, PART, WALSH>()))
+aa_step(StepArgs<T> A, FastDiv div_plane, FastDiv div_lx)
+{
+  using Idx = typename std::conditional<IDX32, unsigned, size_t>::type;
   constexpr int D = (Q == 9) ? 2 : 3;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= A.LX) return;
-  const int j = blockIdx.y, k = blockIdx.z;
-  const int LX = A.LX, LY = A.LY;
-  // Node indices are 32-bit (the host rejects N >= 2^31); direction planes
-  // are reached through 64-bit base pointers, which are uniform per warp.
-  const int plane = LX * LY;
-  const int n = i + LX * j + plane * k;
+  __shared__ Idx sslot[ODD ? Q : 1][256];
+  // Node indices are 32-bit (the host rejects N >= 2^31).
+  const unsigned nu = blockIdx.x * 256u + threadIdx.x;
+  if (nu >= (unsigned)A.N) return;
+  const int n = (int)nu;
   const uint8_t cl = WALSH ? uint8_t(0) : A.cls[n];
   if (cl & CLS_SOLID) return;
-  const uint32_t nb = (cl & CLS_NEAR) ? A.nbm[n] : 0u;
-
-  // dense offsets to the neighbours along each axis (periodic on every
-  // axis, a serial run's wrap); neighbour n + c_a = n + off(a)
-  int xm = (i == 0) ? LX - 1 : -1, xp = (i == LX - 1) ? 1 - LX : 1;
-  int ym = (j == 0) ? plane - LX : -LX, yp = (j == LY - 1) ? LX - plane : LX;
-  int zm = 0, zp = 0;
-  if (D == 3) {
-    const int tot = plane * A.LZ;
-    zm = (k == 0) ? tot - plane : -plane;
-    zp = (k == A.LZ - 1) ? plane - tot : plane;
-  }
-  auto off = [&](int a) -> int {
-    return (cx(a) < 0 ? xm : (cx(a) > 0 ? xp : 0)) + (cy(a) < 0 ? ym : (cy(a) > 0 ? yp : 0))
-         + (cz(a) < 0 ? zm : (cz(a) > 0 ? zp : 0));
-  };
+  const Idx N = (Idx)A.N;
 
   T u[3] = {T(0), T(0), T(0)};
   constexpr int S_BEGIN = (PART == PART_SOLUTE) ? 1 : 0;
@@ -505,28 +521,55 @@ aa_step(StepArgs<T> A)
   for (int s = S_BEGIN; s < S_END; ++s) {
     const bool solute = (NS == 2 && s == 1);
     if (solute && !A.solute_on) break;
-    if (s > 0) {
-      // recompute the solute's neighbour addresses rather than keeping the
-      // flow's live across the flow's collision and push, and start only
-      // after the flow's stores are issued
-      asm volatile("" ::: "memory");
-      xm = opaque(xm); xp = opaque(xp); ym = opaque(ym); yp = opaque(yp);
-      if (D == 3) { zm = opaque(zm); zp = opaque(zp); }
-    }
+    // start the solute only after the flow's stores are issued
+    if (s > 0) asm volatile("" ::: "memory");
     T* const fs = A.f + (size_t)s * Q * (size_t)A.N;
-    const size_t N = (size_t)A.N;
     T d[Q];
     if (ODD) {
       // pull: d_a = f[a][n - c_a], or own f[opp a][n] behind a solid
+      auto pull = [&](int a, Idx src) {
+        sslot[a][threadIdx.x] = src;
+        d[a] = ld_pop(fs + src);
+      };
+      if (s > S_BEGIN) {
+        // the solute's slots are the flow's
 #pragma unroll
-      for (int a = 0; a < Q; ++a) {
-        const size_t src = ((nb >> opp(a)) & 1u) ? (size_t)opp(a) * N + n
-                                                 : (size_t)a * N + (size_t)(n + off(opp(a)));
-        d[a] = fs[src];
+        for (int a = 0; a < Q; ++a) d[a] = ld_pop(fs + sslot[a][threadIdx.x]);
+      } else {
+        // dense offsets to the neighbours along each axis (periodic on
+        // every axis, a serial run's wrap); neighbour n + c_a = n + off(a)
+        const int LX = A.LX, LY = A.LY, plane = LX * LY;
+        const int k = fast_div(n, div_plane);
+        const int r = n - k * plane;
+        const int j = fast_div(r, div_lx);
+        const int i = r - j * LX;
+        const int xm = (i == 0) ? LX - 1 : -1, xp = (i == LX - 1) ? 1 - LX : 1;
+        const int ym = (j == 0) ? plane - LX : -LX, yp = (j == LY - 1) ? LX - plane : LX;
+        int zm = 0, zp = 0;
+        if (D == 3) {
+          const int tot = plane * A.LZ;
+          zm = (k == 0) ? tot - plane : -plane;
+          zp = (k == A.LZ - 1) ? plane - tot : plane;
+        }
+        auto off = [&](int a) -> int {
+          return (cx(a) < 0 ? xm : (cx(a) > 0 ? xp : 0)) + (cy(a) < 0 ? ym : (cy(a) > 0 ? yp : 0))
+               + (cz(a) < 0 ? zm : (cz(a) > 0 ? zp : 0));
+        };
+        // a warp with no node next to a solid forms no selects
+        if (!WALSH && __any_sync(__activemask(), cl & CLS_NEAR)) {
+          const uint32_t nb = (cl & CLS_NEAR) ? A.nbm[n] : 0u;
+#pragma unroll
+          for (int a = 0; a < Q; ++a)
+            pull(a, ((nb >> opp(a)) & 1u) ? (Idx)opp(a) * N + (Idx)n
+                                          : (Idx)a * N + (Idx)(n + off(opp(a))));
+        } else {
+#pragma unroll
+          for (int a = 0; a < Q; ++a) pull(a, (Idx)a * N + (Idx)(n + off(opp(a))));
+        }
       }
     } else {
 #pragma unroll
-      for (int a = 0; a < Q; ++a) d[a] = fs[opp(a) * N + n];
+      for (int a = 0; a < Q; ++a) d[a] = ld_pop(fs + (opp(a) * N + n));
     }
     if (Q == 9 && (cl & (CLS_NORTH | CLS_SOUTH))) {
       T (&d9)[9] = reinterpret_cast<T (&)[9]>(d);
@@ -546,16 +589,10 @@ aa_step(StepArgs<T> A)
       else if (!solute) A.btc[(A.btc_hi - A.btc_lo) + (n - A.btc_lo)] = (double)u[0];
     }
     if (ODD) {
-      // push: f[opp a][n + c_a] = d_a, or own f[a][n] in front of a solid
-      // (offsets laundered so the pull addresses are not kept live)
-      xm = opaque(xm); xp = opaque(xp); ym = opaque(ym); yp = opaque(yp);
-      if (D == 3) { zm = opaque(zm); zp = opaque(zp); }
+      // push: f[opp a][n + c_a] = d_a, or own f[a][n] in front of a solid:
+      // the slot d_opp(a) came from
 #pragma unroll
-      for (int a = 0; a < Q; ++a) {
-        const size_t dst = ((nb >> a) & 1u) ? (size_t)a * N + n
-                                            : (size_t)opp(a) * N + (size_t)(n + off(a));
-        fs[dst] = d[a];
-      }
+      for (int a = 0; a < Q; ++a) fs[sslot[opp(a)][threadIdx.x]] = d[a];
     } else {
       const int n2 = opaque(n);   // do not keep the load addresses live
 #pragma unroll
