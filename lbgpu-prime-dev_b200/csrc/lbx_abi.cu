@@ -217,12 +217,12 @@ void launch_face_nodes(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face
     C.m_skip = f3.lo_end;
     C.m_jump = f3.hi_start - f3.lo_end;
     const long long count = (long long)f3.lo_end + (d->fluid - f3.hi_start);
-    const unsigned blocks = (unsigned)((count + 255) / 256);
-    if (blocks == 0) return;
+    if (count == 0) return;
     const bool idx32 = (unsigned long long)Q * (unsigned long long)d->P < (1ull << 32);
     auto go = [&](auto odd_c, auto idx_c) {
+      constexpr int bs = compact_threads<T, NS, decltype(odd_c)::value, PART_ALL, true>();
       aa_step_compact<T, Q, NS, MODEL, decltype(odd_c)::value, PART_ALL, decltype(idx_c)::value,
-                      false, true><<<blocks, 256, 0, stream>>>(C);
+                      false, true><<<(unsigned)((count + bs - 1) / bs), bs, 0, stream>>>(C);
     };
     using TT = std::true_type;
     using FF = std::false_type;
@@ -232,33 +232,30 @@ void launch_face_nodes(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face
   }
 }
 
-// The step kernels launch_aa uses (an odd step is always one launch, an even
-// step of two substances always two); the others are not compiled.
-template <int NS, int PART, bool ODD>
-constexpr bool step_part_used()
-{
-  return ODD ? PART == PART_ALL : (NS == 1 || PART != PART_ALL);
-}
-
+// One launch over the lattice (compact: over the interior between the
+// z-face planes when f3 is given; launch_face_nodes takes the two planes).
 template <typename T, int Q, int NS, int MODEL, int PART>
-void launch_part(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fused<T>* f3)
+void launch_nodes(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fused<T>* f3)
 {
+  using TT = std::true_type;
+  using FF = std::false_type;
   if (d->layout == LBX_LAYOUT_COMPACT) {
     CompactArgs<T> C = make_compact<T>(d, A);
-    if (f3) {   // the interior only; launch_face_nodes takes the two planes
+    if (f3) {
       C.m_base = f3->lo_end;
       C.m_end = f3->hi_start;
     }
-    const unsigned blocks = (unsigned)((C.m_end - C.m_base + 255) / 256);
-    if (C.m_end <= C.m_base) return;
+    const int count = C.m_end - C.m_base;
+    if (count <= 0) return;
     const bool idx32 = (unsigned long long)Q * (unsigned long long)d->P < (1ull << 32);
     auto go = [&](auto odd_c, auto idx_c, auto oop_c) {
-      if constexpr (step_part_used<NS, PART, decltype(odd_c)::value>())
-        aa_step_compact<T, Q, NS, MODEL, decltype(odd_c)::value, PART, decltype(idx_c)::value,
-                        decltype(oop_c)::value><<<blocks, 256, 0, d->stream>>>(C);
+      constexpr bool o = decltype(odd_c)::value;
+      if constexpr (step_joint<Q, NS, o, true>() == (PART == PART_ALL)) {
+        constexpr int bs = compact_threads<T, NS, o, PART, false>();
+        aa_step_compact<T, Q, NS, MODEL, o, PART, decltype(idx_c)::value, decltype(oop_c)::value>
+            <<<((unsigned)count + bs - 1) / bs, bs, 0, d->stream>>>(C);
+      }
     };
-    using TT = std::true_type;
-    using FF = std::false_type;
     if (A.fout) {
       if (idx32) { if (odd) go(TT{}, TT{}, TT{}); else go(FF{}, TT{}, TT{}); }
       else { if (odd) go(TT{}, FF{}, TT{}); else go(FF{}, FF{}, TT{}); }
@@ -269,16 +266,14 @@ void launch_part(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fused
     d->launches++;
     return;
   }
-  const unsigned blocks = (unsigned)((A.N + 255) / 256);
   const FastDiv dp = make_fastdiv((unsigned)(A.LX * A.LY)), dl = make_fastdiv((unsigned)A.LX);
   const bool idx32 = (unsigned long long)Q * (unsigned long long)A.N < (1ull << 32);
   auto go = [&](auto odd_c, auto idx_c, auto walsh_c) {
-    if constexpr (step_part_used<NS, PART, decltype(odd_c)::value>())
-      aa_step<T, Q, NS, MODEL, decltype(odd_c)::value, PART, decltype(idx_c)::value,
-              decltype(walsh_c)::value><<<blocks, 256, 0, d->stream>>>(A, dp, dl);
+    constexpr bool o = decltype(odd_c)::value;
+    if constexpr (step_joint<Q, NS, o, false>() == (PART == PART_ALL))
+      aa_step<T, Q, NS, MODEL, o, PART, decltype(idx_c)::value, decltype(walsh_c)::value>
+          <<<(unsigned)((A.N + 255) / 256), 256, 0, d->stream>>>(A, dp, dl);
   };
-  using TT = std::true_type;
-  using FF = std::false_type;
   if (A.ns) {
     if (idx32) { if (odd) go(TT{}, TT{}, TT{}); else go(FF{}, TT{}, TT{}); }
     else { if (odd) go(TT{}, FF{}, TT{}); else go(FF{}, FF{}, TT{}); }
@@ -289,12 +284,10 @@ void launch_part(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fused
   d->launches++;
 }
 
-// One step: a single launch for the flow alone; for two substances, an odd
-// step is one launch too (per node the flow, then the solute from the slots
-// the flow's pulls found, its u in registers; written out of place, for the
-// adjoint's recomputation, it also stores u), and an even step is a flow launch that hands u to a solute launch (the solute
-// launch only while the solute is active; fused, the even step spilled and
-// ran slower).
+// One step: one launch, of two substances too where they run jointly
+// (step_joint); else a flow launch that hands u to a solute launch (the
+// solute launch only while the solute is active).  A joint launch written
+// out of place, for the adjoint's recomputation, also stores u.
 // With the z faces fused, the face planes' nodes run in a launch of their
 // own on the side stream, beside the interior launches: in an AA step every
 // node reads and writes only its own set of population slots, the face
@@ -312,13 +305,14 @@ bool launch_aa(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fused<T
     cudaStreamWaitEvent(d->side, d->side_fork, 0);
     launch_face_nodes<T, Q, NS, MODEL>(d, A, odd, *f3, d->side);
   }
-  if constexpr (NS == 1) {
-    launch_part<T, Q, NS, MODEL, PART_ALL>(d, A, odd, f3);
-  } else if (odd) {
-    launch_part<T, Q, NS, MODEL, PART_ALL>(d, A, odd, f3);
-  } else {
-    launch_part<T, Q, NS, MODEL, PART_FLOW>(d, A, odd, f3);
-    if (A.solute_on) launch_part<T, Q, NS, MODEL, PART_SOLUTE>(d, A, odd, f3);
+  const bool compact = d->layout == LBX_LAYOUT_COMPACT;
+  const bool joint = odd ? (compact ? step_joint<Q, NS, true, true>() : step_joint<Q, NS, true, false>())
+                         : (compact ? step_joint<Q, NS, false, true>() : step_joint<Q, NS, false, false>());
+  if (joint) {
+    launch_nodes<T, Q, NS, MODEL, PART_ALL>(d, A, odd, f3);
+  } else if constexpr (NS == 2 && Q == 19) {
+    launch_nodes<T, Q, NS, MODEL, PART_FLOW>(d, A, odd, f3);
+    if (A.solute_on) launch_nodes<T, Q, NS, MODEL, PART_SOLUTE>(d, A, odd, f3);
   }
   if (f3 && !beside) launch_face_nodes<T, Q, NS, MODEL>(d, A, odd, *f3, d->stream);
   return beside;

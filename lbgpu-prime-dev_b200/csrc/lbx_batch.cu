@@ -137,7 +137,7 @@ __device__ __forceinline__ void batch_node(const SampleDesc<T>& S, const BatchAr
   C.div_plane = S.div_plane;
   C.div_lx = S.div_lx;
   C.faces = 0;
-  compact_node<T, Q, 1, MODEL, ODD, PART_ALL, IDX32, false>(C, m);
+  compact_node<T, Q, 1, MODEL, ODD, PART_ALL, IDX32, false, false, 256>(C, m);
 }
 
 // Global-memory path: the block's descriptor from the per-block table, one
@@ -148,10 +148,13 @@ __device__ __forceinline__ void batch_block(const BatchArgs<T>& A, int b)
   batch_node<T, Q, MODEL, ODD, IDX32>(A.blkdesc[b], A, b * blockDim.x + threadIdx.x);
 }
 
+template <typename T, bool ODD>
+constexpr int batch_min_blocks() { return sizeof(T) == 4 ? (ODD ? 6 : 4) : 3; }
+
 // Up to 256 threads per block, resident blocks as for the single-lattice
-// compact kernels.
+// compact kernels (FP64 three).
 template <typename T, int Q, int MODEL, bool ODD, bool IDX32>
-__global__ void __launch_bounds__(256, (compact_min_blocks<T, PART_ALL>()))
+__global__ void __launch_bounds__(256, (batch_min_blocks<T, ODD>()))
 aa_step_batch(BatchArgs<T> A)
 {
   batch_block<T, Q, MODEL, ODD, IDX32>(A, A.block0 + blockIdx.x);
@@ -162,7 +165,7 @@ aa_step_batch(BatchArgs<T> A)
 // in the pool instead cost the odd step 3-6 %: nine dependent constant-cache
 // reads that miss when 512 samples' tables share an SM's constant cache.)
 template <typename T, int Q, int MODEL, bool ODD, bool IDX32>
-__global__ void __launch_bounds__(256, (compact_min_blocks<T, PART_ALL>()))
+__global__ void __launch_bounds__(256, (batch_min_blocks<T, ODD>()))
 aa_step_batch_pool(BatchArgs<T> A, PoolRef R)
 {
   const int bl = R.block0 + blockIdx.x;

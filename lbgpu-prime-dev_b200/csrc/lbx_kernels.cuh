@@ -170,12 +170,19 @@ struct StepArgs {
   double wg[6];
 };
 
-// Which substances one launch of a step kernel advances.  Two-substance
-// steps run as two launches: the flow (PART_FLOW), which also stores its
-// post-force u, then the solute (PART_SOLUTE), which reads it.  One fused
-// body holding both substances needs about twice the registers of either
-// alone (halving occupancy); the split costs 24 B per FP32 node instead.
+// Which substances one launch of a step kernel advances.  Two substances run
+// in one launch (per node the flow, then the solute from the flow's slots
+// with u in registers) where the joint body fits the registers: D2Q9, and
+// the odd step of D3Q19 in the compact layout, where it also saves the
+// second neighbour lookup.  Elsewhere the flow's launch (PART_FLOW) stores
+// its post-force u and the solute's (PART_SOLUTE) reads it.
 enum StepPart { PART_ALL = 0, PART_FLOW = 1, PART_SOLUTE = 2 };
+
+template <int Q, int NS, bool ODD, bool COMPACT>
+__host__ __device__ constexpr bool step_joint()
+{
+  return NS == 1 || Q == 9 || (COMPACT && ODD);
+}
 
 // ---- per-node collision ---------------------------------------------------
 // d[] holds the node's incoming populations of substance s; u carries the
@@ -463,25 +470,25 @@ __device__ __forceinline__ void face_south(int kind, T rho_bc, T rhoA, T drho, b
 // streams periodically with no solid checks (src/lattice.c:2704-2707,
 // :2812-2815); the collision blends by ns (see collide).
 
-// A population load that goes past L1: no thread reads another's slots in
-// the same step, so L1 has nothing to give, and a plain load of a line that
+// A population load, past L1 (CG): no thread reads another's slots in the
+// same step, so L1 has little to give, and a plain load of a line that
 // neighbouring warps store to holds the store up.
-template <typename T>
-__device__ __forceinline__ T ld_pop(const T* p) { return __ldcg(p); }
+template <bool CG, typename T>
+__device__ __forceinline__ T ld_pop(const T* p) { return CG ? __ldcg(p) : *p; }
 
-// Resident 256-thread blocks of the dense kernels: FP32 six (40 registers),
-// FP64 three (80; two substances' solute two, four for D2Q9's 64); the odd
-// step of two substances in one launch as in the compact layout; Walsh
-// kernels hold the incoming populations too.  Measured at 193 x 161 x 120:
-// FP32 odd 105 us at six or five, 109 at four or seven; even 94 us at six,
-// 101 at four; FP64 odd 185 us at three, 221 at two.
+// Resident 256-thread blocks of the dense kernels: FP32 six (40 registers;
+// four with two substances in one thread, five for a solute launch), FP64
+// three (80; four for D2Q9's 64, two with two substances or for a solute
+// launch); Walsh kernels hold the incoming populations too.  Measured at 193 x 161 x 120: FP32 odd 105 us at six or five, 109 at
+// four or seven; even 94 us at six, 101 at four; FP64 odd 185 us at three,
+// 221 at two.
 template <typename T, int Q, int NS, int PART, bool WALSH>
-constexpr int dense_min_blocks()
+__host__ __device__ constexpr int dense_min_blocks()
 {
   return (PART == PART_ALL && NS == 2) ? (sizeof(T) == 4 && !WALSH ? 4 : 2)
+       : PART == PART_SOLUTE           ? (sizeof(T) == 4 ? (WALSH ? 3 : 5) : 2)
        : sizeof(T) == 4                ? (WALSH ? 4 : 6)
-       : WALSH                         ? 2
-                                       : (Q == 9 ? 4 : (PART == PART_SOLUTE ? 2 : 3));
+                                       : (WALSH ? 2 : (Q == 9 ? 4 : 3));
 }
 
 // One thread per node, the nodes numbered through (no block starts anew at
@@ -529,12 +536,12 @@ aa_step(StepArgs<T> A, FastDiv div_plane, FastDiv div_lx)
       // pull: d_a = f[a][n - c_a], or own f[opp a][n] behind a solid
       auto pull = [&](int a, Idx src) {
         sslot[a][threadIdx.x] = src;
-        d[a] = ld_pop(fs + src);
+        d[a] = ld_pop<true>(fs + src);
       };
       if (s > S_BEGIN) {
         // the solute's slots are the flow's
 #pragma unroll
-        for (int a = 0; a < Q; ++a) d[a] = ld_pop(fs + sslot[a][threadIdx.x]);
+        for (int a = 0; a < Q; ++a) d[a] = ld_pop<true>(fs + sslot[a][threadIdx.x]);
       } else {
         // dense offsets to the neighbours along each axis (periodic on
         // every axis, a serial run's wrap); neighbour n + c_a = n + off(a)
@@ -569,7 +576,7 @@ aa_step(StepArgs<T> A, FastDiv div_plane, FastDiv div_lx)
       }
     } else {
 #pragma unroll
-      for (int a = 0; a < Q; ++a) d[a] = ld_pop(fs + (opp(a) * N + n));
+      for (int a = 0; a < Q; ++a) d[a] = ld_pop<true>(fs + (opp(a) * N + n));
     }
     if (Q == 9 && (cl & (CLS_NORTH | CLS_SOUTH))) {
       T (&d9)[9] = reinterpret_cast<T (&)[9]>(d);
@@ -653,42 +660,46 @@ struct CompactArgs {
   int m_base, m_skip, m_jump, m_end;
 };
 
-// Resident 256-thread blocks asked of the compiler: six (40 registers) for
-// the FP32 kernels, where that measured fastest (the solute kernel spills
-// 12-16 bytes there and still runs 4% faster than at three blocks, its
-// natural 85 registers); for FP64 the cap closest above the natural
-// register count (flow 85, solute 128), since a lower cap spills more.
-template <typename T, int PART>
-constexpr int compact_min_blocks()
+// Threads per block and resident blocks asked of the compiler, compact
+// kernels (microseconds of one launch, 256^3 at porosity 0.4 unless said
+// otherwise).  FP32: odd flow six blocks of 256 threads (40 registers; 213,
+// five 222), even four (flow 165 at six, 162 at four; 192 x 192 x 384 at
+// porosity 0.35, flow then solute: 128 + 129 at six, 126 + 125 at four).
+// FP64: odd flow six of 128 (80 registers: 256-thread blocks leave an eighth
+// of the register file idle; 391 -> 375), even three of 256 (307).  Two
+// substances in one thread: odd FP32 192 x 192 x 384 four of 256 (64
+// registers, 313), odd FP64 192^3 four of 128 (346 -> 332); D2Q9 likewise.
+// The z-face planes' nodes (FACES3) are few and their rules need registers:
+// four of 128.
+template <typename T, int NS, bool ODD, int PART, bool FACES3>
+__host__ __device__ constexpr int compact_threads()
 {
-  return sizeof(T) == 4 ? 6 : (PART == PART_SOLUTE ? 2 : 3);
+  return FACES3 || (sizeof(T) == 8 && (ODD || (NS == 2 && PART == PART_ALL))) ? 128 : 256;
 }
 
-// The odd step of two substances in one launch (flow, then the solute from
-// the flow's slot table): four resident blocks (64 registers) in FP32,
-// where it runs without spills (at six blocks it spilled and ran no faster
-// than the two launches it replaces); two (128) in FP64, which spills 4-12
-// bytes there and 230-250 at three blocks.
-template <typename T, int PART, int NS, bool FACES3>
-constexpr int compact_step_min_blocks()
+template <typename T, int NS, bool ODD, int PART, bool FACES3>
+__host__ __device__ constexpr int compact_min_blocks()
 {
-  return (PART == PART_ALL && NS == 2 && !FACES3) ? (sizeof(T) == 4 ? 4 : 2)
-                                                  : compact_min_blocks<T, PART>();
+  if (FACES3 || (NS == 2 && PART == PART_ALL)) return 4;
+  return sizeof(T) == 4 ? (ODD ? 6 : 4) : (ODD ? 6 : 3);
 }
 
 // IDX32: population offsets within one substance's [Q][P] block fit in 32
 // bits (Q * P < 2^32), so slot selects and address arithmetic stay 32-bit.
 // OOP: write the step's result to C.s.fout instead of in place (used to
 // recompute stored forward states for the adjoint).
-// The update of fluid node m (compact index) by one block thread; the
-// odd step's slot table is indexed by threadIdx.x, so a block's threads
-// handle distinct nodes.
+// The update of fluid node m (compact index) by one thread of a block of at
+// most KTHREADS; the odd step's slot table is indexed by threadIdx.x, so a
+// block's threads handle distinct nodes.
+// Loads go past L1 except in the odd steps whose gathered lines neighbouring
+// warps share (FP32 213 against 218 us, FP64 flow 385 against 375).
 template <typename T, int Q, int NS, int MODEL, bool ODD, int PART, bool IDX32, bool OOP,
-          bool FACES3 = false>
+          bool FACES3, int KTHREADS>
 __device__ __forceinline__ void compact_node(const CompactArgs<T>& C, const int m)
 {
   using Idx = typename std::conditional<IDX32, unsigned, size_t>::type;
   constexpr int D = (Q == 9) ? 2 : 3;
+  constexpr bool CG = !ODD || (sizeof(T) == 8 && NS == 1);
   const StepArgs<T>& A = C.s;
   const Idx F = (Idx)C.P;   // plane stride
   const int LX = A.LX, LY = A.LY;
@@ -776,7 +787,7 @@ __device__ __forceinline__ void compact_node(const CompactArgs<T>& C, const int 
     // push reads them here instead of repeating the 18 index lookups;
     // one column per thread, no barrier needed
     // (offsets in the kernel's index type: 64-bit above 2^32 slots)
-    __shared__ Idx sslot[ODD ? Q : 1][256];
+    __shared__ Idx sslot[ODD ? Q : 1][KTHREADS];
     T d[Q];
     if (ODD) {
       // pull: d_a = f[a][idx(n - c_a)], or own f[opp a] behind a solid; the
@@ -784,14 +795,14 @@ __device__ __forceinline__ void compact_node(const CompactArgs<T>& C, const int 
       auto pull = [&](int a, int up) {
         const Idx src = (up >= 0) ? (Idx)a * F + (Idx)up : (Idx)opp(a) * F + (Idx)m;
         sslot[a][threadIdx.x] = src;
-        d[a] = fs[src];
+        d[a] = ld_pop<CG>(fs + src);
       };
-      if (PART == PART_ALL && NS == 2 && s > 0) {
+      if (s > S_BEGIN) {
         // the solute's slots are the flow's (the same solids): read them from
         // the table the flow's pulls filled, this thread's column, instead of
         // repeating the upstream lookups
 #pragma unroll
-        for (int a = 0; a < Q; ++a) d[a] = fs[sslot[a][threadIdx.x]];
+        for (int a = 0; a < Q; ++a) d[a] = ld_pop<CG>(fs + sslot[a][threadIdx.x]);
       } else if (NS == 1) {
         // one lookup per direction: measured faster than the row windows
         // below for the flow-only kernels (0.214 vs 0.218 ms at 256^3 FP32)
@@ -830,7 +841,7 @@ __device__ __forceinline__ void compact_node(const CompactArgs<T>& C, const int 
       }
     } else {
 #pragma unroll
-      for (int a = 0; a < Q; ++a) d[a] = fs[opp(a) * F + m];
+      for (int a = 0; a < Q; ++a) d[a] = ld_pop<CG>(fs + (opp(a) * F + m));
     }
     if constexpr (FACES3 && Q == 19) {
       // z faces: the stand-alone face_plane rules on the loaded populations
@@ -886,13 +897,15 @@ __device__ __forceinline__ void compact_node(const CompactArgs<T>& C, const int 
 
 template <typename T, int Q, int NS, int MODEL, bool ODD, int PART, bool IDX32, bool OOP,
           bool FACES3 = false>
-__global__ void __launch_bounds__(256, (compact_step_min_blocks<T, PART, NS, FACES3>()))
+__global__ void __launch_bounds__((compact_threads<T, NS, ODD, PART, FACES3>()),
+                                  (compact_min_blocks<T, NS, ODD, PART, FACES3>()))
 aa_step_compact(CompactArgs<T> C)
 {
   int m = blockIdx.x * blockDim.x + threadIdx.x + C.m_base;
   if (m >= C.m_skip) m += C.m_jump;
   if (m >= C.m_end) return;
-  compact_node<T, Q, NS, MODEL, ODD, PART, IDX32, OOP, FACES3>(C, m);
+  compact_node<T, Q, NS, MODEL, ODD, PART, IDX32, OOP, FACES3,
+               compact_threads<T, NS, ODD, PART, FACES3>()>(C, m);
 }
 
 // Dense <-> compact exchange of all substances' populations.
