@@ -189,7 +189,8 @@ __host__ __device__ constexpr bool step_joint()
 // fluid velocity to the solute as the reference's per-thread scratch does.
 // sinks: the solute sink applies once on odd steps and twice on even steps
 // (src/k_stream_collide_stream.c:254-256; src/k_collide.c:96-97, :261-262).
-// Returns the node's density (the solute's C), the value stored as rho.
+// Returns the node's density (the solute's C), the value stored as rho;
+// write_mv: store rho and u at node n.
 // WALSH: partial bounce-back with the node's fraction ns (WALSH_NS_ON,
 // src/k_stream_collide_stream.c:129-215, :363-386; src/lattice.c:2936-2939):
 // the momentum is scaled by (1 - ns) before the division, the force term by
@@ -210,10 +211,35 @@ __host__ __device__ constexpr bool step_joint()
 // full clock gains under 1%).  The sums round in another order, which moves
 // FP32 results by a few ulps; FP64, Kahan sums and Walsh runs keep the
 // reference's operation order.
+// Sum of sign(q) v[q] over q with sign(q) in {-1, 0, 1}, in order; starts
+// from the first term, not from 0 (an addition of 0 is not free: it is not
+// the identity on -0, so the compiler keeps it).
+template <int N, typename S, typename T>
+__device__ __forceinline__ T signed_sum(S sign, const T (&v)[N])
+{
+  T r = T(0);
+  bool first = true;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    if (sign(q) == 0) continue;
+    r = first ? (sign(q) > 0 ? v[q] : -v[q]) : (sign(q) > 0 ? add_(r, v[q]) : sub_(r, v[q]));
+    first = false;
+  }
+  return r;
+}
+
+// c_a . u, its terms added in the order x, y, z.
+template <int D, typename T>
+__device__ __forceinline__ T cdotu(int a, const T (&u)[3])
+{
+  return signed_sum<3>([a](int q) { return q == 0 ? cx(a) : (q == 1 ? cy(a) : (D == 3 ? cz(a) : 0)); },
+                       u);
+}
+
 template <int Q, int MODEL>
 __device__ __forceinline__ float collide_pairs(const StepArgs<float>& A, int s, bool solute,
                                                int sinks, float (&d)[Q], float (&u)[3],
-                                               long long n)
+                                               long long n, bool write_mv)
 {
   constexpr int D = (Q == 9) ? 2 : 3;
   constexpr int NP = (Q - 1) / 2;
@@ -229,14 +255,9 @@ __device__ __forceinline__ float collide_pairs(const StepArgs<float>& A, int s, 
     if (sinks == 2) rho *= A.sink1;
     rho *= A.sink1;
   } else {
-    float m0 = 0.f, m1 = 0.f, m2 = 0.f;
-#pragma unroll
-    for (int p = 0; p < NP; ++p) {
-      const int a = 2 * p + 1;
-      if (cx(a) > 0) m0 += dif[p]; else if (cx(a) < 0) m0 -= dif[p];
-      if (cy(a) > 0) m1 += dif[p]; else if (cy(a) < 0) m1 -= dif[p];
-      if (D == 3) { if (cz(a) > 0) m2 += dif[p]; else if (cz(a) < 0) m2 -= dif[p]; }
-    }
+    const float m0 = signed_sum<NP>([](int p) { return cx(2 * p + 1); }, dif);
+    const float m1 = signed_sum<NP>([](int p) { return cy(2 * p + 1); }, dif);
+    const float m2 = D == 3 ? signed_sum<NP>([](int p) { return cz(2 * p + 1); }, dif) : 0.f;
     const float den = (MODEL == SHIFTED_INC) ? c.rhoA
                     : (MODEL == PLAIN_COMP) ? rho : (c.rhoA + rho);
     const float inv = 1.f / den;
@@ -244,20 +265,13 @@ __device__ __forceinline__ float collide_pairs(const StepArgs<float>& A, int s, 
     u[1] = m1 * inv + c.tg[1];
     u[2] = (D == 3) ? m2 * inv + c.tg[2] : 0.f;
   }
-  if (A.write_mv) {
+  if (write_mv) {
     float* m = A.mv + (long long)s * (1 + D) * A.N;
     m[n] = (!solute && MODEL != PLAIN_COMP) ? rho + c.rhoA : rho;
     m[A.N + n] = u[0];
     m[2 * A.N + n] = u[1];
     if (D == 3) m[3 * A.N + n] = u[2];
   }
-  auto cdotu = [&](int a) -> float {
-    float r = 0.f;
-    if (cx(a) > 0) r += u[0]; else if (cx(a) < 0) r -= u[0];
-    if (cy(a) > 0) r += u[1]; else if (cy(a) < 0) r -= u[1];
-    if (D == 3) { if (cz(a) > 0) r += u[2]; else if (cz(a) < 0) r -= u[2]; }
-    return r;
-  };
   if (solute) {
     const float ci = rho * c.itau;
     d[0] = fmaf(d[0], c.omc, wgt<float, Q>(0) * ci);
@@ -265,7 +279,7 @@ __device__ __forceinline__ float collide_pairs(const StepArgs<float>& A, int s, 
     for (int p = 0; p < NP; ++p) {
       const int a = 2 * p + 1;
       const float base = wgt<float, Q>(a) * ci;
-      const float anti = (3.f * base) * cdotu(a);
+      const float anti = (3.f * base) * cdotu<D>(a, u);
       d[a] = fmaf(d[a], c.omc, base + anti);
       d[a + 1] = fmaf(d[a + 1], c.omc, base - anti);
     }
@@ -279,7 +293,7 @@ __device__ __forceinline__ float collide_pairs(const StepArgs<float>& A, int s, 
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       const int a = 2 * p + 1;
-      const float cu = cdotu(a);
+      const float cu = cdotu<D>(a, u);
       const float wq = wgt<float, Q>(a) * qi;
       const float sym = fmaf(wq, fmaf(4.5f * cu, cu, k), wgt<float, Q>(a) * ri);
       const float anti = (3.f * wq) * cu;
@@ -290,18 +304,23 @@ __device__ __forceinline__ float collide_pairs(const StepArgs<float>& A, int s, 
   return rho;
 }
 
-// UNIT_DEN: the caller knows the divisor of the momentum is exactly 1
-// (the shifted incompressible model with rho_A = 1), and m / 1 == m in
-// IEEE arithmetic, so the divisions are left out with the same results.
-template <typename T, int Q, int MODEL, bool WALSH = false, bool UNIT_DEN = false>
+// The reference's operation order (FP64, Kahan sums and Walsh runs).  A pair
+// of opposite directions shares what its two equilibria compute alike: c.u
+// and 3 c.u change sign exactly, 4.5 (c.u)^2 does not change, and c.u is the
+// sum of its non-zero terms (products by 0 and 1 and sums with 0 change no
+// finite value), a quarter fewer FP64 operations, each rounded as before.
+// At 512 threads an SM's FP64 pipe bounds D2Q9's collision: 1416 cycles, 1634
+// with every direction on its own.
+// The momentum is divided by rho_A only where that is not 1 (m / 1 == m).
+template <typename T, int Q, int MODEL, bool WALSH = false>
 __device__ __forceinline__ T collide(const StepArgs<T>& A, int s, bool solute,
                                         int sinks, T (&d)[Q], T (&u)[3],
-                                        long long n)
+                                        long long n, bool write_mv)
 {
   if constexpr (sizeof(T) == 4 && !WALSH) {
     if (!A.kahan)
       return collide_pairs<Q, MODEL>(A, s, solute, sinks, reinterpret_cast<float (&)[Q]>(d),
-                                     reinterpret_cast<float (&)[3]>(u), n);
+                                     reinterpret_cast<float (&)[3]>(u), n, write_mv);
   }
   constexpr int D = (Q == 9) ? 2 : 3;
   const SubsConst<T>& c = A.sc[s];
@@ -332,15 +351,11 @@ __device__ __forceinline__ T collide(const StepArgs<T>& A, int s, bool solute,
     if (sinks == 2) rho *= A.sink1;
     rho *= A.sink1;
   } else {
-    T m0 = T(0), m1 = T(0), m2 = T(0);
-#pragma unroll
-    for (int a = 0; a < Q; ++a) {
-      if (cx(a) > 0) m0 += d[a]; else if (cx(a) < 0) m0 -= d[a];
-      if (cy(a) > 0) m1 += d[a]; else if (cy(a) < 0) m1 -= d[a];
-      if (D == 3) { if (cz(a) > 0) m2 += d[a]; else if (cz(a) < 0) m2 -= d[a]; }
-    }
-    T den = (MODEL == SHIFTED_INC) ? c.rhoA
-          : (MODEL == PLAIN_COMP) ? rho : (c.rhoA + rho);
+    T m0 = signed_sum<Q>([](int a) { return cx(a); }, d);
+    T m1 = signed_sum<Q>([](int a) { return cy(a); }, d);
+    T m2 = D == 3 ? signed_sum<Q>([](int a) { return cz(a); }, d) : T(0);
+    const T den = (MODEL == SHIFTED_INC) ? c.rhoA
+                : (MODEL == PLAIN_COMP) ? rho : (c.rhoA + rho);
     if (WALSH) {
       m0 = (T)__dmul_rn((double)m0, om);
       m1 = (T)__dmul_rn((double)m1, om);
@@ -351,17 +366,18 @@ __device__ __forceinline__ T collide(const StepArgs<T>& A, int s, bool solute,
       u[1] = (T)__dadd_rn((double)(m1 / den), __dmul_rn(ot, A.wg[s * 3 + 1]));
       u[2] = (D == 3) ? (T)__dadd_rn((double)(m2 / den), __dmul_rn(ot, A.wg[s * 3 + 2]))
                       : T(0);
-    } else if (UNIT_DEN) {
+    } else {
+      if (MODEL != SHIFTED_INC || den != T(1)) {
+        m0 = m0 / den;
+        m1 = m1 / den;
+        if (D == 3) m2 = m2 / den;
+      }
       u[0] = add_(m0, c.tg[0]);
       u[1] = add_(m1, c.tg[1]);
       u[2] = (D == 3) ? add_(m2, c.tg[2]) : T(0);
-    } else {
-      u[0] = add_(m0 / den, c.tg[0]);
-      u[1] = add_(m1 / den, c.tg[1]);
-      u[2] = (D == 3) ? add_(m2 / den, c.tg[2]) : T(0);
     }
   }
-  if (A.write_mv) {
+  if (write_mv) {
     T* m = A.mv + (long long)s * (1 + D) * A.N;
     m[n] = (!solute && MODEL != PLAIN_COMP) ? rho + c.rhoA : rho;
     m[A.N + n] = u[0];
@@ -370,27 +386,33 @@ __device__ __forceinline__ T collide(const StepArgs<T>& A, int s, bool solute,
   }
   if (solute) {
     // g_a <- g_a (1 - 1/tau_s) + w_a C (1 + 3 c.u) / tau_s  (src/lattice.c:2858-2875)
+    d[0] = add_(mul_(d[0], c.omc), mul_(mul_(wgt<T, Q>(0), rho), c.itau));
 #pragma unroll
-    for (int a = 0; a < Q; ++a) {
-      T cu = T(cx(a)) * u[0] + T(cy(a)) * u[1] + (D == 3 ? T(cz(a)) * u[2] : T(0));
-      d[a] = add_(mul_(d[a], c.omc),
-                  mul_(mul_(mul_(wgt<T, Q>(a), rho), add_(T(1), mul_(T(3), cu))), c.itau));
+    for (int a = 1; a < Q; a += 2) {
+      const T wr = mul_(wgt<T, Q>(a), rho), cu3 = mul_(T(3), cdotu<D>(a, u));
+      d[a] = add_(mul_(d[a], c.omc), mul_(mul_(wr, add_(T(1), cu3)), c.itau));
+      d[a + 1] = add_(mul_(d[a + 1], c.omc), mul_(mul_(wr, sub_(T(1), cu3)), c.itau));
     }
   } else {
     // BGK in shifted or plain form (src/lattice.c:2880-2919):
     // d (1 - 1/tau) + w drho / tau + w rq (3 cu + 4.5 cu^2 - 1.5 u^2) / tau
     T usq = add_(mul_(u[0], u[0]), mul_(u[1], u[1]));
     if (D == 3) usq = add_(usq, mul_(u[2], u[2]));
-    T rq = (MODEL == SHIFTED_INC) ? c.rhoA
-         : (MODEL == PLAIN_COMP) ? rho : (c.rhoA + rho);
-#pragma unroll
-    for (int a = 0; a < Q; ++a) {
-      // c.u: products by -1, 0, 1 are exact, so contraction cannot change it
-      T cu = T(cx(a)) * u[0] + T(cy(a)) * u[1] + (D == 3 ? T(cz(a)) * u[2] : T(0));
-      T w = wgt<T, Q>(a);
-      T poly = sub_(add_(mul_(T(3), cu), mul_(mul_(T(4.5), cu), cu)), mul_(T(1.5), usq));
+    const T u15 = mul_(T(1.5), usq);
+    const T rq = (MODEL == SHIFTED_INC) ? c.rhoA
+               : (MODEL == PLAIN_COMP) ? rho : (c.rhoA + rho);
+    auto relax = [&](int a, T poly) {
+      const T w = wgt<T, Q>(a);
       d[a] = add_(add_(mul_(d[a], c.omc), mul_(mul_(w, rho), c.itau)),
                   mul_(mul_(mul_(w, rq), poly), c.itau));
+    };
+    relax(0, -u15);
+#pragma unroll
+    for (int a = 1; a < Q; a += 2) {
+      const T cu = cdotu<D>(a, u);
+      const T cu3 = mul_(T(3), cu), cu45 = mul_(mul_(T(4.5), cu), cu);
+      relax(a, sub_(add_(cu3, cu45), u15));
+      relax(a + 1, sub_(sub_(cu45, cu3), u15));
     }
   }
   if (WALSH) {
@@ -586,7 +608,7 @@ aa_step(StepArgs<T> A, FastDiv div_plane, FastDiv div_lx)
       if (cl & CLS_SOUTH)
         face_south<T>(A.face_s[s], A.rho_s[s], A.sc[s].rhoA, A.drho_s[s], shifted, d9);
     }
-    const T rho = collide<T, Q, MODEL, WALSH>(A, s, solute, ODD ? 1 : 2, d, u, n);
+    const T rho = collide<T, Q, MODEL, WALSH>(A, s, solute, ODD ? 1 : 2, d, u, n, A.write_mv);
     if (PART == PART_FLOW && A.solute_on) {
 #pragma unroll
       for (int c = 0; c < D; ++c) A.ubuf[c * A.ustride + n] = u[c];
@@ -869,7 +891,7 @@ __device__ __forceinline__ void compact_node(const CompactArgs<T>& C, const int 
       if (j == 0)
         face_south<T>(A.face_s[s], A.rho_s[s], A.sc[s].rhoA, A.drho_s[s], shifted, d9);
     }
-    const T rho = collide<T, Q, MODEL>(A, s, solute, ODD ? 1 : 2, d, u, n);
+    const T rho = collide<T, Q, MODEL>(A, s, solute, ODD ? 1 : 2, d, u, n, A.write_mv);
     // the flow's u for the solute launch, or, written out of place by the
     // joint launch (the adjoint's recomputation), kept for the adjoint
     if ((PART == PART_FLOW || (PART == PART_ALL && NS == 2 && OOP && s == 0)) && A.solute_on) {

@@ -132,7 +132,7 @@ __device__ __forceinline__ int observe(const int* flag)
 // Step s of a round updates the fluid nodes at distance >= s from the
 // region's edge, from a row-ordered list, so a warp's shared-memory accesses
 // are runs of neighbouring nodes and no lane holds a solid node.
-template <typename T, int MODEL, int K, bool UNIT_DEN>
+template <typename T, int MODEL, int K>
 __global__ void __launch_bounds__(kTiledThreads, 1)
 aa_tiled(StepArgs<T> A, const int* __restrict__ fidx, T* f0, T* f1, long long P, int rounds,
          const int4* __restrict__ plan, int ntiles, const int* __restrict__ nbrs,
@@ -265,7 +265,7 @@ aa_tiled(StepArgs<T> A, const int* __restrict__ fidx, T* f0, T* f1, long long P,
               face_south<T>(A.face_s[0], A.rho_s[0], A.sc[0].rhoA, A.drho_s[0], shifted, d);
           }
           T u[3];
-          collide<T, 9, MODEL, false, UNIT_DEN>(A, 0, false, 1, d, u, 0);
+          collide<T, 9, MODEL>(A, 0, false, 1, d, u, 0, false);
 #pragma unroll
           for (int a = 0; a < 9; ++a) nxt[a * R + node] = d[a];
         }
@@ -434,13 +434,13 @@ lbx_status make_plan(lbx_domain* d, int K)
   return LBX_OK;
 }
 
-template <typename T, int MODEL, bool UNIT_DEN>
+template <typename T, int MODEL>
 lbx_status launch(lbx_domain* d, const StepArgs<T>& A, int rounds)
 {
   constexpr int K = tiled_k<T>();
   static_assert(K % 2 == 0, "a round must end after an even step");
   constexpr size_t smem = tiled_smem<T, K>();
-  const void* fn = (const void*)aa_tiled<T, MODEL, K, UNIT_DEN>;
+  const void* fn = (const void*)aa_tiled<T, MODEL, K>;
   if (d->tiled_grid == 0) {
     int dev = 0, sms = 0, per_sm = 0, coop = 0;
     cudaGetDevice(&dev);
@@ -508,10 +508,9 @@ lbx_status lbx_internal_tiled_run(lbx_domain* d, const StepArgs<T>& A, int round
 {
   if (rounds <= 0) return LBX_OK;
   if (rounds % 2) return lbx_internal_fail(LBX_ERR_INVALID, "tiled rounds must be even");
-  if (d->p.accurate == 0) return launch<T, PLAIN_COMP, false>(d, A, rounds);
-  if (d->p.compressible) return launch<T, SHIFTED_COMP, false>(d, A, rounds);
-  if (A.sc[0].rhoA == T(1)) return launch<T, SHIFTED_INC, true>(d, A, rounds);
-  return launch<T, SHIFTED_INC, false>(d, A, rounds);
+  if (d->p.accurate == 0) return launch<T, PLAIN_COMP>(d, A, rounds);
+  if (d->p.compressible) return launch<T, SHIFTED_COMP>(d, A, rounds);
+  return launch<T, SHIFTED_INC>(d, A, rounds);
 }
 
 template lbx_status lbx_internal_tiled_run<float>(lbx_domain*, const StepArgs<float>&, int);
