@@ -205,14 +205,16 @@ lbx_status lbx_set_stream(lbx_domain* d, void* stream);
 /* How lbx_run advances a stretch of frame-free AA pairs whose launch
  * arguments do not change (no extension of the reference's interface: the
  * reference launches every step, src/lbgpu_prime.cu:517-527, :741-750).
- *   LBX_RUN_AUTO   (default) the tiled path where it applies and the lattice
- *                  is small enough for it to pay, else STEPS;
+ *   LBX_RUN_AUTO   (default) the tiled path where it applies and is the
+ *                  faster one, else STEPS;
  *   LBX_RUN_STEPS  one launch per step, replayed from captured CUDA graphs;
- *   LBX_RUN_TILED  the tiled path wherever it applies: 2D, one substance, no
- *                  Walsh run, no plane record, faces absent or fused.  One
- *                  cooperative launch runs rounds of K steps (K = 6 in FP64,
- *                  10 in FP32) on tiles held in shared memory with halos K
- *                  deep; FP64 results are bit-identical to STEPS.
+ *   LBX_RUN_TILED  the tiled path wherever it applies: 2D, no Walsh run, no
+ *                  plane record, faces absent or fused, a lattice whose
+ *                  tiles fit the GPU's shared memory (about 570^2 nodes in
+ *                  FP64, 800^2 in FP32; with a solute 410^2 and 580^2).  One
+ *                  cooperative launch runs rounds of up to 12 steps on tiles
+ *                  held in shared memory with halos as deep; FP64 results
+ *                  are bit-identical to STEPS.
  * LBX_ERR_INVALID for another mode. */
 enum { LBX_RUN_AUTO = 0, LBX_RUN_STEPS = 1, LBX_RUN_TILED = 2 };
 lbx_status lbx_set_run_mode(lbx_domain* d, int mode);

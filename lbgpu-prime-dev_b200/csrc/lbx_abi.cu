@@ -807,41 +807,31 @@ lbx_status replay_pairs(lbx_domain* d, int t, int pairs)
   return LBX_OK;
 }
 
-// LBX_RUN_AUTO takes the tiled path where every 32 x 16 tile of the
-// lattice can have a block (an SM) of its own: there it beat the per-step
-// path (D2Q9 FP64 128^2 and 256^2: 1.7x and 1.5x); at 512^2 blocks take
-// several tiles each, meet at grid barriers, and lose to it (3x slower).
-bool tiled_applies(const lbx_domain* d)
+// Whether the tiled path takes a stretch of AA pairs starting at odd time t
+// with unchanging arguments; LBX_RUN_AUTO asks its plan whether it is the
+// faster one (lbx_tiled.cu), LBX_RUN_TILED only whether it applies.
+lbx_status tiled_applies(lbx_domain* d, int t, bool* yes)
 {
   const lbx_params& p = d->p;
-  if (d->run_mode == LBX_RUN_STEPS || d->tiled_grid < 0) return false;
-  if (p.dims != 2 || p.nsubs != 1 || d->ns || d->btc_vals || d->fout) return false;
-  if (d->faces_active && !d->faces_fused) return false;
-  if (d->run_mode == LBX_RUN_TILED) return true;
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return (long long)((p.LX + 31) / 32) * ((p.LY + 15) / 16) <= sms;
+  *yes = false;
+  if (d->run_mode == LBX_RUN_STEPS || d->tiled_state < 0) return LBX_OK;
+  if (p.dims != 2 || d->ns || d->btc_vals || d->fout) return LBX_OK;
+  if (d->faces_active && (!d->faces_fused || solute_faces_idle(d, t))) return LBX_OK;
+  bool better = false;
+  if (lbx_status st = lbx_internal_tiled_plan(d, &better)) return st;
+  *yes = d->tiled_state > 0 && (better || d->run_mode == LBX_RUN_TILED);
+  return LBX_OK;
 }
 
-// The tiled path over as many whole, even-numbered rounds as `pairs` AA
-// pairs starting at odd time t hold; returns the pairs it advanced.
-lbx_status tiled_pairs(lbx_domain* d, int t, int pairs, int* done)
+lbx_status tiled_pairs(lbx_domain* d, int t, int pairs, bool write_mv)
 {
-  *done = 0;
-  const int K = lbx_internal_tiled_steps_per_round(d);
-  int rounds = (2 * pairs) / K;
-  rounds -= rounds % 2;
-  if (rounds < 2) return LBX_OK;
   lbx_status st;
-  if (d->real_size == 8) st = lbx_internal_tiled_run<double>(d, make_args<double>(d, t, 0), rounds);
-  else st = lbx_internal_tiled_run<float>(d, make_args<float>(d, t, 0), rounds);
-  if (st != LBX_OK) return st;
-  if (d->layout == LBX_LAYOUT_COMPACT) d->dense_stale = true;
-  *done = rounds * K / 2;
-  return LBX_OK;
+  if (d->real_size == 8)
+    st = lbx_internal_tiled_run<double>(d, make_args<double>(d, t, 0), pairs, write_mv);
+  else
+    st = lbx_internal_tiled_run<float>(d, make_args<float>(d, t, 0), pairs, write_mv);
+  if (st == LBX_OK && d->layout == LBX_LAYOUT_COMPACT) d->dense_stale = true;
+  return st;
 }
 
 // Dense exchange array <-> compact populations.
@@ -921,6 +911,9 @@ lbx_status lbx_create(const lbx_params* p, const uint8_t* solids, lbx_domain** o
                                                                  : LBX_LAYOUT_DENSE)
                   : p->layout;
 
+  // the tiled run's plan reads the mask (lbx_tiled.cu; no larger lattice fits)
+  if (p->dims == 2 && d->N <= (1 << 20)) d->host_solids.assign(solids, solids + d->N);
+
   auto bail = [&](lbx_status s) { release(d); delete d; return s; };
   cudaError_t e;
 #define CKD(call)                                                                  \
@@ -936,7 +929,11 @@ lbx_status lbx_create(const lbx_params* p, const uint8_t* solids, lbx_domain** o
   }
   const size_t fbytes = (size_t)p->nsubs * d->Q * d->N * d->real_size;
   const size_t mvbytes = (size_t)p->nsubs * (1 + d->D) * d->N * d->real_size;
-  CKD(cudaMalloc(&d->f, fbytes));
+  if (d->layout == LBX_LAYOUT_COMPACT) d->P = (d->fluid + 31) / 32 * 32;
+  const size_t tiled_room = p->walsh ? 0 : lbx_internal_tiled_room(d);
+  const size_t tiled_dense = d->layout == LBX_LAYOUT_COMPACT ? 0 : tiled_room;
+  CKD(cudaMalloc(&d->f, (fbytes + 255) / 256 * 256 + tiled_dense));
+  if (tiled_dense) d->tiled_room = (char*)d->f + (fbytes + 255) / 256 * 256;
   CKD(cudaMalloc(&d->mv, mvbytes));
   CKD(cudaMalloc(&d->solids, d->N));
   CKD(cudaMalloc(&d->cls, d->N));
@@ -950,8 +947,9 @@ lbx_status lbx_create(const lbx_params* p, const uint8_t* solids, lbx_domain** o
       if (solids[n] == 1) fidx[n] = -1;
       else { fidx[n] = m; fnode[m++] = (int)n; }
     }
-    d->P = (d->fluid + 31) / 32 * 32;
-    CKD(cudaMalloc(&d->fc, std::max<size_t>(1, (size_t)p->nsubs * d->Q * d->P * d->real_size)));
+    const size_t fcbytes = (size_t)p->nsubs * d->Q * d->P * d->real_size;
+    CKD(cudaMalloc(&d->fc, std::max<size_t>(1, (fcbytes + 255) / 256 * 256 + tiled_room)));
+    if (tiled_room) d->tiled_room = (char*)d->fc + (fcbytes + 255) / 256 * 256;
     CKD(cudaMalloc(&d->fidx, d->N * sizeof(int)));
     CKD(cudaMalloc(&d->fnode, fnode.size() * sizeof(int)));
     CKD(cudaMemcpy(d->fidx, fidx.data(), d->N * sizeof(int), cudaMemcpyHostToDevice));
@@ -1143,30 +1141,34 @@ lbx_status lbx_run(lbx_domain* d, int t0, int nsteps, int frame_rate)
   alignas(16) unsigned char k_odd[kKey], k_even[kKey], k[kKey];
   while (t <= tend) {
     const bool frame = frame_rate > 0 && t % frame_rate == 0;
-    // a stretch of >= 4 frame-free steps starting on an odd time, with the
-    // launch arguments of its first pair throughout, is replayed from a graph
-    if (!frame && (t % 2) == 1 && d->parity == 0 && d->stream != nullptr && tend - t + 1 >= 4) {
+    // a stretch of steps starting on an odd time with the launch arguments
+    // of its first pair throughout: of two or more frame-free pairs it is
+    // replayed from a graph; the tiled run takes a frame's even step with it
+    if (!frame && (t % 2) == 1 && d->parity == 0 && tend - t + 1 >= 4) {
       const size_t ko = step_key(d, t, k_odd), ke = step_key(d, t + 1, k_even);
       int pairs = 0;
+      bool frame_last = false;    // the pair after the frame-free ones ends in a frame
       for (int u = t; u + 1 <= tend; u += 2) {
-        if (frame_rate > 0 && (u % frame_rate == 0 || (u + 1) % frame_rate == 0)) break;
+        if (frame_rate > 0 && u % frame_rate == 0) break;
         if (lbx_internal_pest_due(d, u) || lbx_internal_pest_due(d, u + 1)) break;
-        if (pairs > 0 && (step_key(d, u, k) != ko || std::memcmp(k, k_odd, ko) ||
-                          step_key(d, u + 1, k) != ke || std::memcmp(k, k_even, ke)))
+        if (u > t && (step_key(d, u, k) != ko || std::memcmp(k, k_odd, ko) ||
+                      step_key(d, u + 1, k) != ke || std::memcmp(k, k_even, ke)))
           break;
+        if (frame_rate > 0 && (u + 1) % frame_rate == 0) { frame_last = true; break; }
         ++pairs;
       }
-      if (pairs >= 2) {
-        int done = 0;
-        if (tiled_applies(d)) {
-          if (lbx_status st = tiled_pairs(d, t, pairs, &done)) return st;
-          t += 2 * done;
-          pairs -= done;
-        }
-        if (pairs > 0) {
-          if (lbx_status st = replay_pairs(d, t, pairs)) return st;
-          t += 2 * pairs;
-        }
+      const int all = pairs + (frame_last ? 1 : 0);
+      bool tiled = false;
+      if (all >= 2 && d->stream != nullptr)
+        if (lbx_status st = tiled_applies(d, t, &tiled)) return st;
+      if (tiled) {
+        if (lbx_status st = tiled_pairs(d, t, all, frame_last)) return st;
+        t += 2 * all;
+        continue;
+      }
+      if (pairs >= 2 && d->stream != nullptr) {
+        if (lbx_status st = replay_pairs(d, t, pairs)) return st;
+        t += 2 * pairs;
         continue;
       }
     }

@@ -69,14 +69,22 @@ struct lbx_domain {
   long long graph_launches = 0;          // kernels one replay of the graph runs
   // temporal blocking of small 2D lattices (lbx_tiled.cu)
   int run_mode = LBX_RUN_AUTO;
+  std::vector<uint8_t> host_solids;      // 2D lattices the tiles may fit: the mask, for the plan
+  int tiled_state = 0;                   // 0: not planned, 1: planned, -1: no tiles fit
+  int tiled_k = 0;                       // steps per round, at most
+  double tiled_us = 0.0;                 // modelled time per step
+  void* tiled_room = nullptr;            // memory for the two below, behind the population array
+  void* tiled_own = nullptr;             // or allocated by the plan
   void* tiled_scratch = nullptr;         // a second population array for its rounds
-  int* tiled_flags = nullptr;            // per-tile round counters, then a status word
-  int4* tiled_plan = nullptr;            // per tile: x, y, height
+  void* tiled_plan = nullptr;            // the tiles, then the tables
   int* tiled_nbrs = nullptr;             // per tile: the tiles its halo reads
+  int* tiled_gidx = nullptr;             // per tile: population slots of its region's nodes
+  int* tiled_flags = nullptr;            // per-tile round counters, then a status word
+  unsigned short* tiled_list = nullptr;  // per tile: its node list; then the flags words, the halo list
   int tiled_ntiles = 0;
-  bool tiled_local = false;              // tiles wait for their neighbours only
+  size_t tiled_nodes = 0;                // region nodes of all tiles
   int tiled_base = 0;                    // counter value the next launch starts from
-  int tiled_grid = 0;                    // resident blocks of the tiled kernel (-1: none)
+  bool tiled_attr = false;               // the kernel's shared-memory limit is raised
 };
 
 namespace lbx { template <typename T> struct StepArgs; }
@@ -93,12 +101,18 @@ LBX_HIDDEN void lbx_internal_drop_graphs(lbx_domain* d);
 LBX_HIDDEN bool lbx_internal_pest_due(const lbx_domain* d, int t);
 LBX_HIDDEN lbx_status lbx_internal_pest_after(lbx_domain* d, int t);
 LBX_HIDDEN void lbx_internal_pest_free(lbx_domain* d);
-// Temporal blocking: steps one round advances, and `rounds` (even) rounds
-// with the launch arguments A of every step, from the state after an even
-// step.
-LBX_HIDDEN int lbx_internal_tiled_steps_per_round(const lbx_domain* d);
+// Temporal blocking: plans the tiles on first use (tiled_state tells whether
+// they fit) and tells whether the tiled run is modelled faster than a launch
+// per step; then `pairs` AA pairs (two or more) with the launch arguments A
+// from the state after an even step, the last step writing the macro
+// variables if asked.
+// Bytes the tiled run of this lattice would like behind the population
+// array (0: it would not be taken).
+LBX_HIDDEN size_t lbx_internal_tiled_room(const lbx_domain* d);
+LBX_HIDDEN lbx_status lbx_internal_tiled_plan(lbx_domain* d, bool* better);
 template <typename T>
-LBX_HIDDEN lbx_status lbx_internal_tiled_run(lbx_domain* d, const lbx::StepArgs<T>& A, int rounds);
+LBX_HIDDEN lbx_status lbx_internal_tiled_run(lbx_domain* d, const lbx::StepArgs<T>& A, int pairs,
+                                             bool write_mv);
 LBX_HIDDEN void lbx_internal_tiled_free(lbx_domain* d);
 // LBX_OK, or the error of a tiled launch whose bounded wait ran out (then
 // cleared); synchronous.

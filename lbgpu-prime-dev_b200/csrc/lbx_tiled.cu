@@ -3,111 +3,129 @@
 // A 256 x 256 D2Q9 lattice holds 65k nodes: one step is ~0.3 us of work
 // spread over 148 SMs, and a step launch (or a graph node) costs more than
 // that.  Here one cooperative launch advances the lattice by many steps.
-// The lattice is cut into tiles kTX nodes wide and at most kTYMax high;
-// per round a block loads its tile with a halo of K nodes into shared
-// memory, advances it K steps there (the region still valid shrinks by one
-// node per side per step), and writes the tile's own fluid nodes back.
-// Rounds alternate between the population array and a scratch copy of it,
-// so a round never reads what a slower block of the same round writes.
-// The rounds of one launch are even in number: the state ends in the
-// population array.
+// The lattice is cut into tiles, one block (an SM) each; per round a block
+// loads a halo of up to K nodes around its tile into shared memory, advances
+// the tile K steps there (the region still valid shrinks by one node per
+// side per step), and stores the tile's nodes.  Rounds alternate between the
+// population array and a scratch copy of it, so a round never reads what a
+// slower block of the same round writes.  The rounds of one launch are even
+// in number (the state ends in the population array), of even length each
+// (a round ends after an even step), K steps or fewer: any number of AA
+// pairs from two on is one launch.
 //
-// Tile plan.  Where the columns divide the lattice and every tile gets a
-// block of its own, each column of tiles is cut into heights that give its
-// tiles about equal work per round (fluid node updates, halo included):
-// the slowest tile sets the pace, and the fluid fraction of fixed tiles of
-// a porous lattice spreads from below 0.3 to near 1.  Between rounds a
-// block then waits only for the tiles its halo reads (their round counters,
-// polled by one lane each; the wait is bounded in time and records a
+// Between rounds a block waits only for the tiles its halo reads (their
+// round counters, polled by one lane each; the wait is bounded and records a
 // timeout in a status word the host reads at lbx_sync); a counter at r + 1
 // also means that tile has finished reading the buffer round r + 1 writes.
-// Such a block keeps its tile's nodes in shared memory from round to round
-// (they are valid after K steps), reloads only the halo, and stores only
-// the strip other halos read (every node it owns in the last round).
-// Otherwise the tiles are a fixed grid (the last column may overhang the
-// lattice and wrap onto it), blocks may own several, and rounds meet at a
-// grid barrier.
+// A block keeps its tile's nodes in shared memory from round to round (they
+// are valid after every round), reloads only the halo, and stores only the
+// strip other halos read (every node it owns in the last round).
 //
-// In terms of the post-collision populations g the AA pair is one rule
-// applied twice: after an even step f[a][n] = g_a(n); a step gathers
-// d_a = g_a(n - c_a), or g_opp(a)(n) where n - c_a is solid (the
-// half-way bounce-back of the odd step's pull and of the even step's read
-// of the slot the odd step's push filled), applies the fused Zou-He / zero
-// gradient rows, and collides.  So K steps from the state after an even
-// step (K even) end in the state after an even step, in the same slots, and
+// In shared memory a step is the AA step itself, in place: the odd step
+// pulls d_a from slot a of the upstream node n - c_a (the node's own slot
+// opp(a) behind a solid) and pushes to the slots it pulled from, the even
+// step swaps its own slots.  Every node touches its own slot set only, and
 // the per-node arithmetic is the step kernels' own (collide, face_north,
-// face_south): FP64 results are bit-identical to the per-step path.
+// face_south): FP64 results are bit-identical to the per-step path.  A step
+// in place needs one population buffer where pulling from one buffer into
+// another needs two, which is what lets two substances (the flow, then the
+// solute from the flow's slots with u in registers) or larger tiles fit.
+// The last step can write the macro variables (a frame's step).
 //
-// Eligible: 2D, one substance, no Walsh run, no plane record, faces absent
-// or fused, a run of AA pairs whose launch arguments do not change (what
-// the graph replay needs too).
+// Tile plan (host).  Columns of about equal width, each cut into heights of
+// about equal work per round (fluid node updates, halo included): the
+// slowest tile sets the pace, and the fluid fraction of fixed tiles of a
+// porous lattice spreads from below 0.3 to near 1.  Width, rows per column
+// and K come from a small cost model (see best_shapes).  The tiles' node
+// tables are made once, on the device (tile_tables), and read by every
+// launch: made anew in each launch they cost 15-20 us, more than the 20
+// steps between two frames of a small lattice.
+//
+// Eligible: 2D, no Walsh run, no plane record, faces absent or fused, a run
+// of AA pairs whose launch arguments do not change (what the graph replay
+// needs too).
 #include "lbx.h"
 #include "lbx_internal.h"
 #include "lbx_kernels.cuh"
 
-#include <cooperative_groups.h>
-
 #include <algorithm>
+#include <cmath>
+#include <cstring>
 #include <vector>
 
-namespace cg = cooperative_groups;
 using namespace lbx;
 
 namespace {
 
-constexpr int kTX = 32;                // tile width
-constexpr int kTYMax = 16;             // tile height, at most
 constexpr int kTiledThreads = 512;
-constexpr int kMaxNb = 32;             // tiles one halo may read (one warp polls them)
+constexpr int kMaxNb = 64;             // tiles one halo may read (one warp polls them)
+constexpr int kMaxK = 12;              // steps per round, at most
 constexpr long long kWaitLimit = 1LL << 20;   // polls of one counter (about a second)
 
-// Steps per round: FP64 six (a halo six nodes deep), FP32 ten (its nodes
-// take half the shared memory); measured best of 4/6 and 6/8/10.
-template <typename T>
-constexpr int tiled_k() { return sizeof(T) == 8 ? 6 : 10; }
+// Region nodes (tile and halo) a block holds in its 227 KB: Q populations
+// per substance, a slot index, two list entries and a flags word per node.
+template <typename T, int NS>
+__host__ __device__ constexpr int tiled_cap()
+{
+  return (227 * 1024 - 1024) / (NS * 9 * (int)sizeof(T) + 10) / 32 * 32;
+}
 
-// A tile's node lists (tile-local node indices of fluid nodes, row order),
-// by the node's distance e from the edge of the tile's region:
-//   kListAll    every fluid node (the first load)
-//   kListHalo   e < K: the halo, reloaded every round
-//   kListStrip  K <= e < 2K: the tile's nodes other halos read
-//   kListStep + s (s = 1..K)  e >= s: the nodes step s of a round updates;
-//               s = K: the tile's own nodes
-constexpr int kListAll = 0, kListHalo = 1, kListStrip = 2, kListStep = 2;
-
-template <int K>
-__host__ __device__ constexpr int tiled_region() { return (kTX + 2 * K) * (kTYMax + 2 * K); }
-
-template <typename T, int K>
+template <typename T, int NS>
 constexpr size_t tiled_smem()
 {
-  constexpr int R = tiled_region<K>();
-  return 2 * 9 * R * sizeof(T) + R * sizeof(int) + (4 + K) * R * sizeof(unsigned short);
+  return (size_t)tiled_cap<T, NS>() * (NS * 9 * sizeof(T) + 10);
 }
+
+// Row pitch of a tile's region: odd, so that the nodes of a column (the
+// halo's sides in list order) lie in different banks (256^2 FP64, K = 8: 2.4
+// us per step; at the even pitch of 48 3.3).
+__host__ __device__ constexpr int tiled_pitch(int w, int K) { return (w + 2 * K) | 1; }
+
+// One tile: its lattice rectangle and the bounds of its node list.  The list
+// holds the region's fluid nodes (region-local indices, tiled_pitch) in
+// the order: interior (at least 2K from the region's edge), strip (the
+// tile's other nodes, which other halos read), then the halo's rings from
+// the innermost out, each part in row order; step j of a round of k steps
+// updates the nodes at least K - k + j from the edge, a prefix of the list.
+// A second list holds the halo's nodes in row order, for loading it: by
+// rings, the halo's sides put every lane of a load in a line of its own
+// (256^2 FP64, K = 6: 2.1 us against 1.2).
+struct Tile {
+  int x, y, w, h;
+  int at;                     // where its tables begin
+  int interior, own;          // nodes in the interior; in the tile
+  int ring[kMaxK + 1];        // ring[j]: nodes through the j innermost rings (ring[0] = own)
+};
 
 // A region node's flags word: bit a (a < 9) the node upstream in direction
 // a (n - c_a) is solid; kWSolid the node itself is solid; kWNorth / kWSouth
 // its class bits.
 constexpr unsigned kWSolid = 1u << 15, kWNorth = 1u << 9, kWSouth = 1u << 10;
 
-// Exclusive prefix sum of one flag per thread over the block; *total gets
-// the sum.  `warp_sums` holds kTiledThreads / 32 ints.
-__device__ __forceinline__ int block_scan(bool flag, int* warp_sums, int* total)
+template <typename T>
+struct TiledArgs {
+  T* f0;                        // the population array [nsubs][9][P] (dense: P = N)
+  T* f1;                        // scratch of the same shape
+  long long P;
+  const Tile* tiles;
+  // per tile from Tile::at on, an entry per region node:
+  const int* gidx;              // population slot
+  const unsigned short* list;
+  const unsigned short* wrd;    // flags words
+  const unsigned short* halo;   // the halo's nodes by rows
+  const int* nbrs;              // [ntiles][kMaxNb]: the tiles a halo reads, -1 after the last
+  int* flags;                   // per-tile round counters
+  int* status;
+  int base;                     // counter value this launch starts from
+  int K;
+  int pairs, rounds;            // AA pairs spread over the (even) number of rounds
+  int write_mv;                 // the last step writes the macro variables
+};
+
+// Steps of round r: the pairs spread evenly, the first rounds one longer.
+__device__ __forceinline__ int round_steps(int pairs, int rounds, int r)
 {
-  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const unsigned ball = __ballot_sync(0xffffffffu, flag);
-  const int in_warp = __popc(ball & ((1u << lane) - 1u));
-  if (lane == 0) warp_sums[warp] = __popc(ball);
-  __syncthreads();
-  int before = 0, all = 0;
-  for (int w = 0; w < kTiledThreads / 32; ++w) {
-    const int c = warp_sums[w];
-    if (w < (int)warp) before += c;
-    all += c;
-  }
-  __syncthreads();
-  *total = all;
-  return before + in_warp;
+  return 2 * (pairs / rounds + (r < pairs % rounds ? 1 : 0));
 }
 
 // Round counters: tile t has stored the strips of round r when
@@ -125,407 +143,638 @@ __device__ __forceinline__ int observe(const int* flag)
   return v;
 }
 
-// f0: the population array (dense [Q][N] or compact [Q][P]); f1: scratch
-// of the same shape; fidx: dense -> compact (null for the dense layout).
-// plan[t] = (x, y, height) of tile t; nbrs[t][0..kMaxNb): the tiles its
-// halo reads, -1 after the last (local waits only).
-// Step s of a round updates the fluid nodes at distance >= s from the
-// region's edge, from a row-ordered list, so a warp's shared-memory accesses
-// are runs of neighbouring nodes and no lane holds a solid node.
-template <typename T, int MODEL, int K>
-__global__ void __launch_bounds__(kTiledThreads, 1)
-aa_tiled(StepArgs<T> A, const int* __restrict__ fidx, T* f0, T* f1, long long P, int rounds,
-         const int4* __restrict__ plan, int ntiles, const int* __restrict__ nbrs,
-         int local_waits, int* flags, int base, int* status)
+// One node's update in shared memory (b: [NS][9][cap]) at parity ODD.
+template <typename T, int NS, int MODEL, bool ODD>
+__device__ __forceinline__ void tiled_node(const StepArgs<T>& A, T* b, int node, unsigned w,
+                                           int pitch, bool write_mv, int n)
 {
-  constexpr int RX = kTX + 2 * K, R = tiled_region<K>();
-  constexpr int NL = 3 + K;
-  static_assert(R < 65536, "tile list entries are 16-bit");
-  extern __shared__ __align__(16) unsigned char smem[];
-  T* const b0 = reinterpret_cast<T*>(smem);            // [9][R]
-  T* const b1 = b0 + 9 * R;                             // [9][R]
-  int* const gidx = reinterpret_cast<int*>(b1 + 9 * R); // [R]: slot of the node, -1 solid
-  unsigned short* const lists = reinterpret_cast<unsigned short*>(gidx + R);  // [NL][R]
-  unsigned short* const wrd = lists + NL * R;                                // [R] flags words
-  __shared__ int warp_sums[kTiledThreads / 32];
-  __shared__ int lcount[NL];
-  __shared__ int gave_up;
-  cg::grid_group grid = cg::this_grid();
-  const int LX = A.LX, LY = A.LY;
-  const bool keep = ntiles <= (int)gridDim.x;          // one tile per block
-  const bool shifted = MODEL != PLAIN_COMP;
-  bool tables = false;
-  int4 g = keep ? plan[blockIdx.x] : make_int4(0, 0, 0, 0);
+  constexpr int cap = tiled_cap<T, NS>();
+  int slot[9];                  // where d_a is read; d_opp(a) is written there
+#pragma unroll
+  for (int a = 0; a < 9; ++a) {
+    if (ODD) {
+      const int up = node - (cy(a) < 0 ? -pitch : (cy(a) > 0 ? pitch : 0)) - cx(a);
+      slot[a] = ((w >> a) & 1u) ? opp(a) * cap + node : a * cap + up;
+    } else {
+      slot[a] = opp(a) * cap + node;
+    }
+  }
+  T u[3] = {T(0), T(0), T(0)};
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    if (s == 1 && !A.solute_on) break;
+    T* const fs = b + s * 9 * cap;
+    T d[9];
+#pragma unroll
+    for (int a = 0; a < 9; ++a) d[a] = fs[slot[a]];
+    if (w & (kWNorth | kWSouth)) {
+      const bool shifted = MODEL != PLAIN_COMP && s == 0;
+      if (w & kWNorth)
+        face_north<T>(A.face_n[s], A.rho_n[s], A.sc[s].rhoA, A.drho_n[s], shifted, d);
+      if (w & kWSouth)
+        face_south<T>(A.face_s[s], A.rho_s[s], A.sc[s].rhoA, A.drho_s[s], shifted, d);
+    }
+    collide<T, 9, MODEL>(A, s, s == 1, ODD ? 1 : 2, d, u, n, write_mv);
+#pragma unroll
+    for (int a = 0; a < 9; ++a) fs[slot[opp(a)]] = d[a];
+  }
+}
 
-  for (int r = 0; r < rounds; ++r) {
-    const T* const src = (r & 1) ? f1 : f0;
-    T* const dst = (r & 1) ? f0 : f1;
-    if (local_waits && r > 0) {
-      // this block's tile is blockIdx.x; lane q of warp 0 waits for the q-th
-      // tile its halo reads to finish round r - 1
+// Block t advances tile t by all rounds.  Lists keep a warp's shared-memory
+// accesses runs of neighbouring nodes with no lane on a solid node.
+template <typename T, int NS, int MODEL>
+__global__ void __launch_bounds__(kTiledThreads, 1)
+aa_tiled(StepArgs<T> A, TiledArgs<T> R)
+{
+  constexpr int cap = tiled_cap<T, NS>();
+  extern __shared__ __align__(16) unsigned char smem[];
+  T* const b = reinterpret_cast<T*>(smem);                                  // [NS][9][cap]
+  int* const gidx = reinterpret_cast<int*>(b + NS * 9 * cap);               // [cap]
+  unsigned short* const list = reinterpret_cast<unsigned short*>(gidx + cap);
+  unsigned short* const wrd = list + cap;
+  unsigned short* const halo = wrd + cap;
+  __shared__ Tile tile;
+  __shared__ int gave_up;
+  const int K = R.K;
+  if (threadIdx.x < sizeof(Tile) / 4)
+    reinterpret_cast<int*>(&tile)[threadIdx.x] =
+        reinterpret_cast<const int*>(R.tiles + blockIdx.x)[threadIdx.x];
+  __syncthreads();
+  const int pitch = tiled_pitch(tile.w, K), region = pitch * (tile.h + 2 * K);
+  const size_t at = (size_t)tile.at;
+  for (int i = threadIdx.x; i < region; i += kTiledThreads) {
+    gidx[i] = R.gidx[at + i];
+    list[i] = R.list[at + i];
+    wrd[i] = R.wrd[at + i];
+    halo[i] = R.halo[at + i];
+  }
+  __syncthreads();
+  const int subs = (NS == 2 && A.solute_on) ? 2 : 1;
+
+  for (int r = 0; r < R.rounds; ++r) {
+    const T* const src = (r & 1) ? R.f1 : R.f0;
+    T* const dst = (r & 1) ? R.f0 : R.f1;
+    const int k = round_steps(R.pairs, R.rounds, r);
+    if (r > 0) {
+      // lane q of warp 0 waits for the q-th (and the 32 + q-th) tile the halo
+      // reads to finish round r - 1
       if (threadIdx.x < 32) {
         int late = 0;
-        const int nb = nbrs[blockIdx.x * kMaxNb + threadIdx.x];
-        if (nb >= 0) {
+#pragma unroll 1
+        for (int q = threadIdx.x; q < kMaxNb && !late; q += 32) {
+          const int nb = R.nbrs[blockIdx.x * kMaxNb + q];
+          if (nb < 0) break;
           long long polls = 0;
           // every poll is an L2 round trip: no sleep between polls
-          while (observe(flags + nb) < base + r) {
-            if (++polls >= kWaitLimit || *(volatile int*)status != 0) { late = 1; break; }
+          while (observe(R.flags + nb) < R.base + r) {
+            if (++polls >= kWaitLimit || *(volatile int*)R.status != 0) { late = 1; break; }
           }
         }
         late = __any_sync(0xffffffffu, late);
         if (threadIdx.x == 0) {
-          if (late) atomicExch(status, 1);
+          if (late) atomicExch(R.status, 1);
           gave_up = late;
         }
       }
       __syncthreads();
       if (gave_up) return;          // every thread of the block leaves together
     }
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-      if (!keep) g = plan[tile];
-      const int x0 = g.x - K, y0 = g.y - K, RY = g.z + 2 * K, RR = RX * RY;
-      __syncthreads();                                  // the last tile's stores read smem
-      if (!(keep && tables)) {
-        for (int i = threadIdx.x; i < RR; i += kTiledThreads) {
-          int gx = (x0 + i % RX) % LX, gy = (y0 + i / RX) % LY;
-          if (gx < 0) gx += LX;
-          if (gy < 0) gy += LY;
-          const int n = gx + LX * gy;
-          const uint8_t c = A.cls[n];
-          wrd[i] = (unsigned short)(((c & CLS_SOLID) ? kWSolid : 0u) | ((c & CLS_NORTH) ? kWNorth : 0u) |
-                                    ((c & CLS_SOUTH) ? kWSouth : 0u));
-          gidx[i] = (c & CLS_SOLID) ? -1 : (fidx ? fidx[n] : n);
-        }
-        __syncthreads();
-        // upstream solid bits of the nodes a step can update (e >= 1)
-        for (int i = threadIdx.x; i < RR; i += kTiledThreads) {
-          const int lx = i % RX, ly = i / RX;
-          if (lx < 1 || lx > RX - 2 || ly < 1 || ly > RY - 2 || (wrd[i] & kWSolid)) continue;
-          unsigned bits = 0;
+    // the tile's own nodes once, the halo every round, all of a node's loads
+    // in flight together (two nodes a thread at a time spilled and lost)
+    auto load = [&](const unsigned short* nodes, int count) {
+      for (int q = threadIdx.x; q < count; q += kTiledThreads) {
+        const int i = nodes[q];
+        const T* const g = src + gidx[i];
+        T v[NS][9];
 #pragma unroll
-          for (int a = 0; a < 9; ++a)
-            if (wrd[i - (cx(a) + RX * cy(a))] & kWSolid) bits |= 1u << a;
-          wrd[i] |= (unsigned short)bits;
-        }
-        __syncthreads();
-        for (int l = 0; l < NL; ++l) {
-          int cnt = 0;
-          for (int c0 = 0; c0 < RR; c0 += kTiledThreads) {
-            const int i = c0 + threadIdx.x;
-            bool flag = false;
-            if (i < RR && !(wrd[i] & kWSolid)) {
-              const int lx = i % RX, ly = i / RX;
-              const int e = min(min(lx, RX - 1 - lx), min(ly, RY - 1 - ly));
-              flag = l == kListAll || (l == kListHalo && e < K) ||
-                     (l == kListStrip && e >= K && e < 2 * K) ||
-                     (l > kListStep && e >= l - kListStep);
-            }
-            int tot;
-            const int pos = block_scan(flag, warp_sums, &tot);
-            if (flag) lists[l * R + cnt + pos] = (unsigned short)i;
-            cnt += tot;
+        for (int s = 0; s < NS; ++s)
+          if (s < subs) {
+#pragma unroll
+            for (int a = 0; a < 9; ++a) v[s][a] = __ldcg(g + (s * 9 + a) * R.P);
           }
-          if (threadIdx.x == 0) lcount[l] = cnt;
-        }
-        __syncthreads();
-      }
-      {
-        const int l = (keep && tables) ? kListHalo : kListAll;
-        const unsigned short* const L = lists + l * R;
-        const int cnt = lcount[l];
-        for (int q = threadIdx.x; q < cnt; q += kTiledThreads) {
-          const int i = L[q];
-          const int m = gidx[i];
 #pragma unroll
-          for (int a = 0; a < 9; ++a) b0[a * R + i] = __ldcg(src + a * P + m);
-        }
+        for (int s = 0; s < NS; ++s)
+          if (s < subs) {
+#pragma unroll
+            for (int a = 0; a < 9; ++a) b[(s * 9 + a) * cap + i] = v[s][a];
+          }
       }
-      tables = true;
-      __syncthreads();
-      T* cur = b0;
-      T* nxt = b1;
+    };
+    if (r == 0) load(list, tile.own);
+    load(halo, tile.ring[K] - tile.own);
+    __syncthreads();
+    const bool last = r + 1 == R.rounds;
 #pragma unroll 1
-      for (int s = 1; s <= K; ++s) {
-        const unsigned short* const L = lists + (kListStep + s) * R;
-        const int cnt = lcount[kListStep + s];
-        for (int q = threadIdx.x; q < cnt; q += kTiledThreads) {
-          const int node = L[q];
-          const unsigned w = wrd[node];
-          T d[9];
-#pragma unroll
-          for (int a = 0; a < 9; ++a) {
-            const int up = node - (cx(a) + RX * cy(a));
-            d[a] = ((w >> a) & 1u) ? cur[opp(a) * R + node] : cur[a * R + up];
-          }
-          if (w & (kWNorth | kWSouth)) {
-            if (w & kWNorth)
-              face_north<T>(A.face_n[0], A.rho_n[0], A.sc[0].rhoA, A.drho_n[0], shifted, d);
-            if (w & kWSouth)
-              face_south<T>(A.face_s[0], A.rho_s[0], A.sc[0].rhoA, A.drho_s[0], shifted, d);
-          }
-          T u[3];
-          collide<T, 9, MODEL>(A, 0, false, 1, d, u, 0, false);
-#pragma unroll
-          for (int a = 0; a < 9; ++a) nxt[a * R + node] = d[a];
-        }
-        __syncthreads();
-        T* const x = cur; cur = nxt; nxt = x;
+    for (int j = 1; j <= k; j += 2) {
+      const int n_odd = tile.ring[k - j], n_even = tile.ring[k - j - 1];
+      for (int q = threadIdx.x; q < n_odd; q += kTiledThreads) {
+        const int node = list[q];
+        tiled_node<T, NS, MODEL, true>(A, b, node, wrd[node], pitch, false, 0);
       }
-      // K is even: the round's result is in b0 (cur)
-      {
-        const bool all = !keep || !local_waits || r + 1 == rounds;
-        const int l = all ? kListStep + K : kListStrip;
-        const unsigned short* const L = lists + l * R;
-        const int cnt = lcount[l];
-        for (int q = threadIdx.x; q < cnt; q += kTiledThreads) {
-          const int node = L[q];
-          if (x0 + node % RX >= LX || y0 + node / RX >= LY) continue;   // overhanging tiles
-          const int m = gidx[node];
-#pragma unroll
-          for (int a = 0; a < 9; ++a) dst[a * P + m] = cur[a * R + node];
+      __syncthreads();
+      const bool mv = last && j + 1 == k && R.write_mv;
+      for (int q = threadIdx.x; q < n_even; q += kTiledThreads) {
+        const int node = list[q];
+        int n = 0;
+        if (mv) {                   // an own node: inside the lattice
+          const int ly = node / pitch, lx = node - ly * pitch;
+          n = (tile.x + lx - K) + A.LX * (tile.y + ly - K);
         }
+        tiled_node<T, NS, MODEL, false>(A, b, node, wrd[node], pitch, mv, n);
+      }
+      __syncthreads();
+    }
+    for (int q = (last ? 0 : tile.interior) + threadIdx.x; q < tile.own; q += kTiledThreads) {
+      const int i = list[q];
+      const int m = gidx[i];
+      for (int s = 0; s < subs; ++s) {
+        T* const g = dst + (size_t)s * 9 * R.P + m;
+#pragma unroll
+        for (int a = 0; a < 9; ++a) g[a * R.P] = b[(s * 9 + a) * cap + i];
       }
     }
-    if (r + 1 < rounds) {
-      if (local_waits) {
-        __syncthreads();                                // the block's stores are issued
-        if (threadIdx.x == 0) publish(flags + blockIdx.x, base + r + 1);
-      } else {
-        grid.sync();
-      }
+    if (!last) {
+      __syncthreads();              // the block's stores are issued
+      if (threadIdx.x == 0) publish(R.flags + blockIdx.x, R.base + r + 1);
     }
   }
 }
+
+// The node tables of tile blockIdx.x (Tile's list bounds included).  Warp c
+// gathers list part c: interior, strip, ring K-1, ..., ring 0; warp K+2 the
+// halo by rows.
+__global__ void __launch_bounds__(kTiledThreads)
+tile_tables(const uint8_t* cls, const int* fidx, int LX, int LY, int K, Tile* tiles, int* gidx,
+            unsigned short* list, unsigned short* wrd, unsigned short* halo)
+{
+  extern __shared__ unsigned short w[];             // [cap] flags words
+  __shared__ int count[kTiledThreads / 32];
+  Tile& t = tiles[blockIdx.x];
+  const int width = t.w + 2 * K, pitch = tiled_pitch(t.w, K), rows = t.h + 2 * K;
+  const int region = pitch * rows;
+  const int x0 = t.x - K, y0 = t.y - K;
+  const size_t at = (size_t)t.at;
+  for (int i = threadIdx.x; i < region; i += kTiledThreads) {
+    if (i % pitch >= width) {                       // the pitch's padding
+      w[i] = (unsigned short)kWSolid;
+      gidx[at + i] = -1;
+      continue;
+    }
+    int gx = (x0 + i % pitch) % LX, gy = (y0 + i / pitch) % LY;
+    if (gx < 0) gx += LX;
+    if (gy < 0) gy += LY;
+    const int n = gx + LX * gy;
+    const uint8_t c = cls[n];
+    w[i] = (unsigned short)(((c & CLS_SOLID) ? kWSolid : 0u) | ((c & CLS_NORTH) ? kWNorth : 0u) |
+                            ((c & CLS_SOUTH) ? kWSouth : 0u));
+    gidx[at + i] = (c & CLS_SOLID) ? -1 : (fidx ? fidx[n] : n);
+  }
+  __syncthreads();
+  // upstream solid bits of the nodes a step can update (off the region's edge)
+  for (int i = threadIdx.x; i < region; i += kTiledThreads) {
+    const int lx = i % pitch, ly = i / pitch;
+    unsigned bits = w[i];
+    if (lx >= 1 && lx <= width - 2 && ly >= 1 && ly <= rows - 2 && !(bits & kWSolid)) {
+#pragma unroll
+      for (int a = 1; a < 9; ++a)
+        if (w[i - (cx(a) + pitch * cy(a))] & kWSolid) bits |= 1u << a;
+    }
+    wrd[at + i] = (unsigned short)bits;
+  }
+  const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto in_part = [&](int i) -> bool {
+    if (i >= region || (w[i] & kWSolid)) return false;
+    const int lx = i % pitch, ly = i / pitch;
+    const int e = min(min(lx, width - 1 - lx), min(ly, rows - 1 - ly));
+    if (part == K + 2) return e < K;
+    return part == 0 ? e >= 2 * K : (part == 1 ? e >= K && e < 2 * K : e == K + 1 - part);
+  };
+  int mine = 0;
+  if (part < K + 2)
+    for (int i = lane; i - lane < region; i += 32)
+      mine += __popc(__ballot_sync(0xffffffffu, in_part(i)));
+  if (lane == 0) count[part] = mine;
+  __syncthreads();
+  int pos = 0;
+  for (int c = 0; c < part; ++c) pos += count[c];
+  if (part < K + 2 && lane == 0) {
+    if (part == 0) t.interior = pos + mine;
+    else if (part == 1) t.own = t.ring[0] = pos + mine;
+    else t.ring[part - 1] = pos + mine;
+  }
+  if (part == K + 2) pos = 0;
+  unsigned short* const out = part == K + 2 ? halo : list;
+  if (part < K + 3)
+    for (int i = lane; i - lane < region; i += 32) {
+      const bool f = in_part(i);
+      const unsigned ball = __ballot_sync(0xffffffffu, f);
+      if (f) out[at + pos + __popc(ball & ((1u << lane) - 1u))] = (unsigned short)i;
+      pos += __popc(ball);
+    }
+}
+static_assert(kMaxK + 3 <= kTiledThreads / 32, "a warp per list part");
 
 // ---- the tile plan (host) ---------------------------------------------------
 
 // Fluid counts over rectangles of the periodic lattice, halos included.
 struct FluidSums {
-  int LX, LY, ext;
+  int LX, LY, ext, W;
   std::vector<int> s;   // prefix sums over [-ext, LY + ext) x [-ext, LX + ext)
 
   FluidSums(const std::vector<uint8_t>& solids, int lx, int ly, int e)
-      : LX(lx), LY(ly), ext(e), s((size_t)(ly + 2 * e + 1) * (lx + 2 * e + 1), 0)
+      : LX(lx), LY(ly), ext(e), W(lx + 2 * e + 1), s((size_t)(ly + 2 * e + 1) * W, 0)
   {
-    const int W = LX + 2 * ext + 1;
-    for (int y = 0; y < LY + 2 * ext; ++y)
+    std::vector<int> gx(LX + 2 * ext);
+    for (int x = 0; x < LX + 2 * ext; ++x) gx[x] = ((x - ext) % LX + LX) % LX;
+    for (int y = 0; y < LY + 2 * ext; ++y) {
+      const uint8_t* row = solids.data() + (size_t)LX * (((y - ext) % LY + LY) % LY);
+      const int* above = &s[(size_t)y * W];
+      int* here = &s[(size_t)(y + 1) * W];
+      int sum = 0;
       for (int x = 0; x < LX + 2 * ext; ++x) {
-        const int gx = ((x - ext) % LX + LX) % LX, gy = ((y - ext) % LY + LY) % LY;
-        const int f = solids[(size_t)gx + (size_t)LX * gy] != 1;
-        s[(size_t)(y + 1) * W + x + 1] = f + s[(size_t)y * W + x + 1] + s[(size_t)(y + 1) * W + x] -
-                                         s[(size_t)y * W + x];
+        sum += row[gx[x]] != 1;
+        here[x + 1] = above[x + 1] + sum;
       }
+    }
   }
   // fluid nodes in [x0, x1) x [y0, y1), -ext <= x0 <= x1 <= LX + ext (same for y)
   int rect(int x0, int y0, int x1, int y1) const
   {
-    const int W = LX + 2 * ext + 1;
     x0 += ext; x1 += ext; y0 += ext; y1 += ext;
     return s[(size_t)y1 * W + x1] - s[(size_t)y0 * W + x1] - s[(size_t)y1 * W + x0] +
            s[(size_t)y0 * W + x0];
   }
-  // node updates of one round of a tile (x0, y0, h): steps 1..K
-  long long work(int x0, int y0, int h, int K) const
+  // fluid nodes within j of the tile (x0, y0, w, h)
+  long long around(int x0, int y0, int w, int h, int j) const
   {
-    long long w = 0;
-    for (int st = 1; st <= K; ++st)
-      w += rect(x0 - K + st, y0 - K + st, x0 + kTX + K - st, y0 + h + K - st);
-    return w;
+    return rect(x0 - j, y0 - j, x0 + w + j, y0 + h + j);
+  }
+  // node updates of one round of a tile, about: the sum of around(j) over
+  // j = 0 .. K - 1 by Simpson's rule (exact where the fluid is uniform)
+  long long work(int x0, int y0, int w, int h, int K) const
+  {
+    return K * (around(x0, y0, w, h, 0) + 4 * around(x0, y0, w, h, (K - 1) / 2) +
+                around(x0, y0, w, h, K - 1)) / 6;
   }
 };
 
-struct TilePlan {
-  std::vector<int4> tiles;
-  std::vector<int> nbrs;   // [tiles][kMaxNb]
-  bool local = false;
+struct Shape {
+  int cols, rows, K;
+  int tiles;            // at most this many; denser columns get more of them
+  double us;            // modelled time per step
 };
 
-// Equal-work columns (see the file comment); false when they do not apply.
-bool equal_work_plan(const std::vector<uint8_t>& solids, int LX, int LY, int K, int blocks,
-                     TilePlan& out)
+// Modelled microseconds per step.  A step costs a latency and its node
+// updates; a round adds its boundary, a latency (counters, fence, store) and
+// the halo's load.  Steps fitted to clock spans: 256^2 FP64 (tiles 32 x 9) a
+// step of 261 nodes 0.75 us, of 690 1.3; FP32 of 256 nodes 0.34, of 950
+// 0.93; 300 x 220 FP64 with a solute of 346 nodes 1.1, of 700 1.9.  The
+// boundary to whole runs (modelled / measured, us per step): 256^2 FP64
+// K = 8 1.9 / 1.8, 400^2 FP64 K = 6 3.1 / 3.1, 560^2 FP64 K = 2 5.3 / 5.6,
+// 512^2 FP32 K = 6 2.8 / 2.6, 48 x 67 FP64 K = 8 1.2 / 1.2.
+template <typename T, int NS>
+double shape_us(double fluid, int w, int h, int K)
 {
-  if (LX % kTX != 0) return false;
-  const int cols = LX / kTX;
-  if ((long long)cols * ((LY + kTYMax - 1) / kTYMax) > blocks) return false;
-  const FluidSums fs(solids, LX, LY, K + kTYMax);
-  auto cut = [&](long long W, std::vector<int4>* tiles) {
-    long long n = 0;
-    for (int c = 0; c < cols; ++c) {
-      for (int y = 0; y < LY;) {
-        int h = 1;
-        while (h < kTYMax && y + h < LY && fs.work(c * kTX, y, h + 1, K) <= W) ++h;
-        if (tiles) tiles->push_back(make_int4(c * kTX, y, h, 0));
-        y += h;
-        ++n;
+  const double lat = sizeof(T) == 8 ? 0.37 : 0.13;
+  const double node = (sizeof(T) == 8 ? 1.4e-3 : 0.8e-3) * (NS == 2 ? 1.65 : 1.0);
+  // the round's node updates: (w + 2 j)(h + 2 j) over j = 0 .. K - 1
+  const double k = K, area = (double)w * h;
+  const double nodes = k * area + (w + h) * k * (k - 1) + 2. / 3. * k * (k - 1) * (2 * k - 1);
+  return (4.0 + 6.2e-3 * NS * fluid * ((w + 2 * k) * (h + 2 * k) - area) + node * fluid * nodes) / k +
+         lat;
+}
+
+// The launch-per-step path's: a launch and the populations, from the L2
+// (FP64 2.4 us for 2k fluid nodes, 2.9 for 39k, 3.7 for 104k, 5.7 for 227k;
+// 3.7 for 43k with a solute; FP32 2.5 for 39k, 4.1 for 170k).
+double steps_us(double nodes, size_t real, int nsubs)
+{
+  return 2.3 + nodes * nsubs * (real == 8 ? 1.5e-5 : 1.2e-5);
+}
+
+// The shapes whose regions fit a block and whose tiles fit the SMs: the best
+// few, best first.
+constexpr int kShapes = 8;
+
+template <typename T, int NS>
+int best_shapes(int LX, int LY, double fluid, int blocks, Shape (&best)[kShapes])
+{
+  int n = 0;
+  for (int cols = 1; cols <= std::min(LX, blocks); ++cols) {
+    const int w = (LX + cols - 1) / cols;
+    for (int rows = 1, last = 0; rows <= std::min(LY, blocks / cols); ++rows) {
+      const int h = (LY + rows - 1) / rows;
+      if (h == last && rows != blocks / cols) continue;     // the same tiles
+      last = h;
+      for (int K = 2; K <= kMaxK; K += 2) {
+        if (tiled_pitch(w, K) * (h + 2 * K) > tiled_cap<T, NS>()) break;
+        // tiles a halo reads, about: their heights vary
+        const int nx = std::min(cols, 2 * ((K + w - 1) / w) + 1);
+        const int ny = std::min(rows, 2 * ((K + h - 1) / h) + 1);
+        if (nx * ny > kMaxNb / 2) continue;
+        const int tiles = rows == blocks / cols ? blocks : cols * rows;
+        const Shape sh = {cols, rows, K, tiles, shape_us<T, NS>(fluid, w, h, K)};
+        int at = n;
+        while (at > 0 && sh.us < best[at - 1].us) --at;
+        if (at == kShapes) continue;
+        if (n < kShapes) ++n;
+        for (int i = n - 1; i > at; --i) best[i] = best[i - 1];
+        best[at] = sh;
       }
     }
-    return n;
+  }
+  return n;
+}
+
+// Tiles of about equal work for a shape; false when a halo reads too many.
+bool make_tiles(const FluidSums& fs, int LX, int LY, const Shape& sh, int cap,
+                std::vector<Tile>& tiles, std::vector<int>& nbrs)
+{
+  const int K = sh.K;
+  auto edge = [&](int c) { return (int)((long long)LX * c / sh.cols); };
+  auto cut = [&](long long W, std::vector<Tile>* to) -> bool {
+    int n = 0;
+    for (int c = 0; c < sh.cols && n <= sh.tiles; ++c) {
+      const int x = edge(c), w = edge(c + 1) - x;
+      const int hmax = cap / tiled_pitch(w, K) - 2 * K;
+      for (int y = 0; y < LY && n <= sh.tiles; ++n) {
+        int h = 1;
+        while (h < hmax && y + h < LY && fs.work(x, y, w, h + 1, K) <= W) ++h;
+        if (to) {
+          Tile t;
+          std::memset(&t, 0, sizeof t);
+          t.x = x; t.y = y; t.w = w; t.h = h;
+          to->push_back(t);
+        }
+        y += h;
+      }
+    }
+    return n <= sh.tiles;
   };
-  long long lo = 0, hi = 0;
-  for (int c = 0; c < cols; ++c)
-    for (int y = 0; y < LY; y += kTYMax)
-      hi = std::max(hi, fs.work(c * kTX, y, std::min(kTYMax, LY - y), K));
-  while (lo < hi) {               // the least work bound that needs at most `blocks` tiles
+  // about the least work bound that needs no more tiles (to 2 %)
+  long long hi = 0;
+  for (int c = 0; c < sh.cols; ++c)
+    hi += fs.work(edge(c), 0, edge(c + 1) - edge(c), (LY + sh.rows - 1) / sh.rows, K);
+  hi = hi / sh.cols + 1;
+  long long lo = 0;
+  while (!cut(hi, nullptr)) {
+    if (hi > (1LL << 40)) return false;
+    lo = hi;
+    hi *= 2;
+  }
+  while (hi - lo > 1 + hi / 50) {
     const long long mid = (lo + hi) / 2;
-    if (cut(mid, nullptr) <= blocks) hi = mid; else lo = mid + 1;
+    if (cut(mid, nullptr)) hi = mid; else lo = mid;
   }
-  out.tiles.clear();
-  cut(lo, &out.tiles);
-  // the tiles each halo reads
-  std::vector<int> owner((size_t)LX * LY);
-  for (size_t t = 0; t < out.tiles.size(); ++t) {
-    const int4 g = out.tiles[t];
-    for (int y = g.y; y < g.y + g.z; ++y)
-      for (int x = g.x; x < g.x + kTX; ++x) owner[(size_t)x + (size_t)LX * y] = (int)t;
-  }
-  out.nbrs.assign(out.tiles.size() * kMaxNb, -1);
-  for (size_t t = 0; t < out.tiles.size(); ++t) {
-    const int4 g = out.tiles[t];
+  tiles.clear();
+  cut(hi, &tiles);
+  // the tiles each halo reads: its columns, each looked at once per row
+  std::vector<int> column(LX), owner((size_t)sh.cols * LY);
+  for (int c = 0; c < sh.cols; ++c)
+    for (int x = edge(c); x < edge(c + 1); ++x) column[x] = c;
+  for (size_t t = 0; t < tiles.size(); ++t)
+    for (int y = tiles[t].y; y < tiles[t].y + tiles[t].h; ++y)
+      owner[(size_t)column[tiles[t].x] * LY + y] = (int)t;
+  nbrs.assign(tiles.size() * kMaxNb, -1);
+  std::vector<int> cols;
+  for (size_t t = 0; t < tiles.size(); ++t) {
+    const Tile& g = tiles[t];
+    cols.clear();
+    for (int x = g.x - K; x < g.x + g.w + K; ++x) {
+      const int c = column[(x % LX + LX) % LX];
+      if (cols.empty() || cols.back() != c) cols.push_back(c);
+    }
     int k = 0;
-    int* const row = &out.nbrs[t * kMaxNb];
-    for (int y = g.y - K; y < g.y + g.z + K; ++y)
-      for (int x = g.x - K; x < g.x + kTX + K; ++x) {
-        const int o = owner[(size_t)((x % LX + LX) % LX) + (size_t)LX * ((y % LY + LY) % LY)];
+    int* const row = &nbrs[t * kMaxNb];
+    for (int c : cols)
+      for (int y = g.y - K, last = -1; y < g.y + g.h + K; ++y) {
+        const int o = owner[(size_t)c * LY + (y % LY + LY) % LY];
+        if (o == last) continue;
+        last = o;
         if (std::find(row, row + k, o) != row + k) continue;
         if (k == kMaxNb) return false;
         row[k++] = o;
       }
   }
-  out.local = true;
   return true;
 }
 
-TilePlan fixed_plan(int LX, int LY)
+// Region nodes of a shape's tiles, at most (heights sum to LY per column).
+size_t region_nodes(const Shape& sh, int LX, int LY)
 {
-  TilePlan p;
-  for (int y = 0; y < LY; y += kTYMax)
-    for (int x = 0; x < LX; x += kTX)
-      p.tiles.push_back(make_int4(x, y, std::min(kTYMax, LY - y), 0));
-  p.nbrs.assign(p.tiles.size() * kMaxNb, -1);
-  return p;
+  return (size_t)tiled_pitch((LX + sh.cols - 1) / sh.cols, sh.K) *
+         ((size_t)sh.cols * LY + (size_t)sh.tiles * 2 * sh.K);
 }
 
-lbx_status make_plan(lbx_domain* d, int K)
+// Bytes of a plan's scratch array, and of its tables: tiles, neighbours,
+// counters and status, then per region node a slot and three list entries.
+size_t scratch_bytes(const lbx_domain* d)
 {
-  std::vector<uint8_t> solids((size_t)d->N);
-  cudaError_t e = cudaMemcpy(solids.data(), d->solids, (size_t)d->N, cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return lbx_internal_fail(LBX_ERR_CUDA, cudaGetErrorString(e));
-  TilePlan p;
-  if (!equal_work_plan(solids, d->p.LX, d->p.LY, K, d->tiled_grid, p))
-    p = fixed_plan(d->p.LX, d->p.LY);
-  const int nt = (int)p.tiles.size();
-  e = cudaMalloc(&d->tiled_plan, (size_t)nt * sizeof(int4));
-  if (e == cudaSuccess) e = cudaMalloc(&d->tiled_nbrs, p.nbrs.size() * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc(&d->tiled_flags, (size_t)(nt + 1) * sizeof(int));
+  const long long P = d->layout == LBX_LAYOUT_COMPACT ? d->P : d->N;
+  return ((size_t)d->p.nsubs * 9 * P * d->real_size + 255) / 256 * 256;
+}
+
+size_t tables_bytes(int tiles, size_t nodes)
+{
+  return (size_t)tiles * (sizeof(Tile) + (kMaxNb + 1) * sizeof(int)) + sizeof(int) +
+         nodes * (sizeof(int) + 3 * sizeof(unsigned short));
+}
+
+template <typename T, int NS>
+size_t room(const lbx_domain* d, int blocks)
+{
+  Shape shapes[kShapes];
+  const double fluid = (double)d->fluid / (double)d->N;
+  const int n = best_shapes<T, NS>(d->p.LX, d->p.LY, fluid, blocks, shapes);
+  if (n == 0 || shapes[0].us >= steps_us((double)d->fluid, d->real_size, NS)) return 0;
+  size_t most = 0;
+  for (int i = 0; i < n; ++i)
+    most = std::max(most, tables_bytes(shapes[i].tiles, region_nodes(shapes[i], d->p.LX, d->p.LY)));
+  return scratch_bytes(d) + most;
+}
+
+// Plans the lattice's tiles and makes their tables, once per domain:
+// tiled_state 1, or -1 where no shape fits; it stays 0 where one fits but
+// the launch-per-step path is modelled faster and the run mode does not ask.
+template <typename T, int NS>
+lbx_status make_plan(lbx_domain* d)
+{
+  const lbx_params& p = d->p;
+  d->tiled_state = -1;
+  int sms = 0, coop = 0;
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, p.device);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device);
+  if (!coop || sms < 1 || d->fluid == 0) { cudaGetLastError(); return LBX_OK; }
+  const double fluid = (double)d->fluid / (double)d->N;
+  Shape shapes[kShapes];
+  const int ns = best_shapes<T, NS>(p.LX, p.LY, fluid, sms, shapes);
+  // not worth a plan unless some run mode would take it
+  if (ns == 0 || (d->run_mode != LBX_RUN_TILED &&
+                  shapes[0].us >= steps_us((double)d->fluid, d->real_size, p.nsubs))) {
+    d->tiled_state = ns == 0 ? -1 : 0;
+    return LBX_OK;
+  }
+  const FluidSums fs(d->host_solids, p.LX, p.LY, kMaxK);
+  constexpr int cap = tiled_cap<T, NS>();
+  std::vector<Tile> tiles;
+  std::vector<int> nbrs;
+  int i = 0;
+  while (i < ns && !make_tiles(fs, p.LX, p.LY, shapes[i], cap, tiles, nbrs)) ++i;
+  if (i == ns) return LBX_OK;
+  const int nt = (int)tiles.size();
+  d->tiled_k = shapes[i].K;
+  d->tiled_us = shapes[i].us;
+  d->tiled_ntiles = nt;
+  d->tiled_base = 0;
+  size_t nodes = 0;
+  for (Tile& t : tiles) {
+    t.at = (int)nodes;
+    nodes += (size_t)tiled_pitch(t.w, d->tiled_k) * (t.h + 2 * d->tiled_k);
+  }
+  const size_t b_tiles = (size_t)nt * sizeof(Tile), b_nbrs = nbrs.size() * sizeof(int);
+  const size_t b_flags = (size_t)(nt + 1) * sizeof(int), b_gidx = nodes * sizeof(int);
+  std::vector<char> head(b_tiles + b_nbrs + b_flags, 0);   // counters and status start at 0
+  std::memcpy(head.data(), tiles.data(), b_tiles);
+  std::memcpy(head.data() + b_tiles, nbrs.data(), b_nbrs);
+  // the scratch array, then the tables: behind the population array where
+  // lbx_create left room (a call here costs 0.4 ms), else on their own
+  const size_t scratch = scratch_bytes(d);
+  cudaError_t e = cudaSuccess;
+  if (!d->tiled_room) {
+    e = cudaMalloc(&d->tiled_own, scratch + tables_bytes(nt, nodes));
+    d->tiled_room = d->tiled_own;
+  }
+  d->tiled_scratch = d->tiled_room;
+  char* at = (char*)d->tiled_room + scratch;
+  d->tiled_plan = at;
+  d->tiled_nbrs = (int*)(at + b_tiles);
+  d->tiled_flags = (int*)(at + b_tiles + b_nbrs);
+  d->tiled_gidx = (int*)(at + b_tiles + b_nbrs + b_flags);
+  d->tiled_list = (unsigned short*)(at + b_tiles + b_nbrs + b_flags + b_gidx);
+  d->tiled_nodes = nodes;
   if (e == cudaSuccess)
-    e = cudaMemcpy(d->tiled_plan, p.tiles.data(), (size_t)nt * sizeof(int4), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(d->tiled_nbrs, p.nbrs.data(), p.nbrs.size() * sizeof(int), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(d->tiled_flags, 0, (size_t)(nt + 1) * sizeof(int));
+    e = cudaMemcpyAsync(at, head.data(), head.size(), cudaMemcpyHostToDevice, d->stream);
+  if (e == cudaSuccess) {
+    tile_tables<<<nt, kTiledThreads, (size_t)cap * sizeof(unsigned short), d->stream>>>(
+        d->cls, d->layout == LBX_LAYOUT_COMPACT ? d->fidx : nullptr, p.LX, p.LY, d->tiled_k,
+        (Tile*)d->tiled_plan, d->tiled_gidx, d->tiled_list, d->tiled_list + nodes,
+        d->tiled_list + 2 * nodes);
+    d->launches++;
+    e = cudaGetLastError();
+  }
   if (e != cudaSuccess) {
     lbx_internal_tiled_free(d);
+    d->tiled_state = -1;
     return lbx_internal_fail(e == cudaErrorMemoryAllocation ? LBX_ERR_NOMEM : LBX_ERR_CUDA,
                              cudaGetErrorString(e));
   }
-  d->tiled_ntiles = nt;
-  d->tiled_local = p.local;
-  d->tiled_base = 0;
+  d->tiled_state = 1;
   return LBX_OK;
 }
 
-template <typename T, int MODEL>
-lbx_status launch(lbx_domain* d, const StepArgs<T>& A, int rounds)
+template <typename T, int NS, int MODEL>
+lbx_status launch(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
 {
-  constexpr int K = tiled_k<T>();
-  static_assert(K % 2 == 0, "a round must end after an even step");
-  constexpr size_t smem = tiled_smem<T, K>();
-  const void* fn = (const void*)aa_tiled<T, MODEL, K>;
-  if (d->tiled_grid == 0) {
-    int dev = 0, sms = 0, per_sm = 0, coop = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kTiledThreads, smem);
-    if (e != cudaSuccess || !coop || per_sm < 1) {
-      cudaGetLastError();
-      d->tiled_grid = -1;
-    } else {
-      d->tiled_grid = sms * per_sm;
-    }
+  constexpr size_t smem = tiled_smem<T, NS>();
+  const void* fn = (const void*)aa_tiled<T, NS, MODEL>;
+  const int nt = d->tiled_ntiles;
+  // an even number of rounds of at most tiled_k steps, two at least
+  const int per = d->tiled_k / 2;
+  const int rounds = std::max(2, ((pairs + per - 1) / per + 1) / 2 * 2);
+  cudaError_t e = cudaSuccess;
+  if (!d->tiled_attr) {
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return lbx_internal_fail(LBX_ERR_CUDA, cudaGetErrorString(e));
+    d->tiled_attr = true;
   }
-  if (d->tiled_grid < 0) return lbx_internal_fail(LBX_ERR_CUDA, "tiled run unavailable on this device");
-  const bool compact = d->layout == LBX_LAYOUT_COMPACT;
-  const long long P = compact ? d->P : d->N;
-  if (!d->tiled_scratch) {
-    cudaError_t e = cudaMalloc(&d->tiled_scratch, (size_t)9 * P * sizeof(T));
-    if (e != cudaSuccess)
-      return lbx_internal_fail(e == cudaErrorMemoryAllocation ? LBX_ERR_NOMEM : LBX_ERR_CUDA,
-                               "tiled scratch allocation failed");
-  }
-  if (!d->tiled_plan)
-    if (lbx_status st = make_plan(d, K)) return st;
-  const int ntiles = d->tiled_ntiles;
   if (d->tiled_base + rounds + 1 >= (1 << 30)) {
     // restart the counters before they could wrap
-    cudaError_t e = cudaMemsetAsync(d->tiled_flags, 0, (size_t)ntiles * sizeof(int), d->stream);
+    e = cudaMemsetAsync(d->tiled_flags, 0, (size_t)nt * sizeof(int), d->stream);
     if (e != cudaSuccess) return lbx_internal_fail(LBX_ERR_CUDA, cudaGetErrorString(e));
     d->tiled_base = 0;
   }
+  const bool compact = d->layout == LBX_LAYOUT_COMPACT;
   StepArgs<T> a = A;
-  const int* fidx = compact ? d->fidx : nullptr;
-  T* f0 = (T*)(compact ? d->fc : d->f);
-  T* f1 = (T*)d->tiled_scratch;
-  long long pp = P;
-  const int4* plan = d->tiled_plan;
-  int nt = ntiles;
-  const int* nbrs = d->tiled_nbrs;
-  int local = d->tiled_local ? 1 : 0;
-  int* flags = d->tiled_flags;
-  int* status = d->tiled_flags + ntiles;
-  int base = d->tiled_base;
-  void* args[] = {&a, &fidx, &f0, &f1, &pp, &rounds, &plan, &nt, &nbrs, &local, &flags, &base, &status};
-  const int grid = std::min(d->tiled_grid, ntiles);
-  cudaError_t e = cudaLaunchCooperativeKernel(fn, grid, kTiledThreads, args, smem, d->stream);
-  if (e != cudaSuccess)
-    return lbx_internal_fail(LBX_ERR_CUDA, cudaGetErrorString(e));
+  TiledArgs<T> r;
+  r.f0 = (T*)(compact ? d->fc : d->f);
+  r.f1 = (T*)d->tiled_scratch;
+  r.P = compact ? d->P : d->N;
+  r.tiles = (const Tile*)d->tiled_plan;
+  r.gidx = d->tiled_gidx;
+  r.list = d->tiled_list;
+  r.wrd = r.list + d->tiled_nodes;
+  r.halo = r.wrd + d->tiled_nodes;
+  r.nbrs = d->tiled_nbrs;
+  r.flags = d->tiled_flags;
+  r.status = d->tiled_flags + nt;
+  r.base = d->tiled_base;
+  r.K = d->tiled_k;
+  r.pairs = pairs;
+  r.rounds = rounds;
+  r.write_mv = write_mv ? 1 : 0;
+  void* args[] = {&a, &r};
+  e = cudaLaunchCooperativeKernel(fn, nt, kTiledThreads, args, smem, d->stream);
+  if (e != cudaSuccess) return lbx_internal_fail(LBX_ERR_CUDA, cudaGetErrorString(e));
   d->tiled_base += rounds;
   d->launches++;
   return LBX_OK;
 }
 
+template <typename T, int NS>
+lbx_status run_ns(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
+{
+  if (d->p.accurate == 0) return launch<T, NS, PLAIN_COMP>(d, A, pairs, write_mv);
+  if (d->p.compressible) return launch<T, NS, SHIFTED_COMP>(d, A, pairs, write_mv);
+  return launch<T, NS, SHIFTED_INC>(d, A, pairs, write_mv);
+}
+
 }  // namespace
 
-int lbx_internal_tiled_steps_per_round(const lbx_domain* d)
+size_t lbx_internal_tiled_room(const lbx_domain* d)
 {
-  return d->real_size == 8 ? tiled_k<double>() : tiled_k<float>();
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->p.device) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (d->fluid == 0 || d->host_solids.empty()) return 0;
+  if (d->real_size == 8) return d->p.nsubs == 2 ? room<double, 2>(d, sms) : room<double, 1>(d, sms);
+  return d->p.nsubs == 2 ? room<float, 2>(d, sms) : room<float, 1>(d, sms);
+}
+
+lbx_status lbx_internal_tiled_plan(lbx_domain* d, bool* better)
+{
+  const lbx_params& p = d->p;
+  *better = false;
+  if (d->tiled_state == 0 && !d->host_solids.empty()) {
+    lbx_status st = d->real_size == 8
+                        ? (p.nsubs == 2 ? make_plan<double, 2>(d) : make_plan<double, 1>(d))
+                        : (p.nsubs == 2 ? make_plan<float, 2>(d) : make_plan<float, 1>(d));
+    if (st != LBX_OK) return st;
+  }
+  *better = d->tiled_state > 0 &&
+            d->tiled_us < steps_us((double)d->fluid, d->real_size, p.nsubs);
+  return LBX_OK;
 }
 
 template <typename T>
-lbx_status lbx_internal_tiled_run(lbx_domain* d, const StepArgs<T>& A, int rounds)
+lbx_status lbx_internal_tiled_run(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
 {
-  if (rounds <= 0) return LBX_OK;
-  if (rounds % 2) return lbx_internal_fail(LBX_ERR_INVALID, "tiled rounds must be even");
-  if (d->p.accurate == 0) return launch<T, PLAIN_COMP>(d, A, rounds);
-  if (d->p.compressible) return launch<T, SHIFTED_COMP>(d, A, rounds);
-  return launch<T, SHIFTED_INC>(d, A, rounds);
+  if (pairs < 2 || d->tiled_state <= 0)
+    return lbx_internal_fail(LBX_ERR_INVALID, "tiled run without a plan or two pairs");
+  return d->p.nsubs == 2 ? run_ns<T, 2>(d, A, pairs, write_mv) : run_ns<T, 1>(d, A, pairs, write_mv);
 }
 
-template lbx_status lbx_internal_tiled_run<float>(lbx_domain*, const StepArgs<float>&, int);
-template lbx_status lbx_internal_tiled_run<double>(lbx_domain*, const StepArgs<double>&, int);
+template lbx_status lbx_internal_tiled_run<float>(lbx_domain*, const StepArgs<float>&, int, bool);
+template lbx_status lbx_internal_tiled_run<double>(lbx_domain*, const StepArgs<double>&, int, bool);
 
 void lbx_internal_tiled_free(lbx_domain* d)
 {
-  cudaFree(d->tiled_scratch);
-  cudaFree(d->tiled_flags);
-  cudaFree(d->tiled_plan);
-  cudaFree(d->tiled_nbrs);
-  d->tiled_scratch = nullptr;
-  d->tiled_flags = nullptr;
-  d->tiled_plan = nullptr;
-  d->tiled_nbrs = nullptr;
+  if (d->tiled_own) { cudaFree(d->tiled_own); d->tiled_room = nullptr; }
+  d->tiled_own = d->tiled_plan = d->tiled_scratch = nullptr;
+  d->tiled_nbrs = d->tiled_gidx = d->tiled_flags = nullptr;
+  d->tiled_list = nullptr;
+  d->tiled_state = 0;
 }
 
 lbx_status lbx_internal_tiled_status(lbx_domain* d)

@@ -410,7 +410,7 @@ class Domain:
         """How run() advances stretches of AA pairs with unchanging launch
         arguments: "auto" (default), "steps" (a launch per step, replayed
         from CUDA graphs) or "tiled" (temporal blocking in shared memory,
-        2D one-substance lattices; see lbx_set_run_mode in lbx.h)."""
+        small 2D lattices; see lbx_set_run_mode in lbx.h)."""
         if mode not in self.RUN_MODES:
             raise ValueError("run mode must be one of %s" % sorted(self.RUN_MODES))
         _check(_lib.lbx_set_run_mode(self._h, self.RUN_MODES[mode]))
