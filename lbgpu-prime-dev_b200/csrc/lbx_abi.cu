@@ -1000,6 +1000,7 @@ lbx_status lbx_create(const lbx_params* p, const uint8_t* solids, lbx_domain** o
   CKD(cudaGetLastError());
   CKD(cudaStreamSynchronize(d->stream));
 #undef CKD
+  lbx_internal_copy_user(p->device, 1);
   *out = d;
   return LBX_OK;
 }
@@ -1009,6 +1010,7 @@ lbx_status lbx_destroy(lbx_domain* d)
   if (!d) return LBX_OK;
   if (d->stream) cudaStreamSynchronize(d->stream);
   release(d);
+  lbx_internal_copy_user(d->p.device, -1);
   delete d;
   return LBX_OK;
 }
@@ -1024,8 +1026,7 @@ lbx_status lbx_upload_f(lbx_domain* d, int subs, const void* f_host)
   if (d->dense_stale && d->p.nsubs > 1) {
     if (lbx_status st = exchange(d, false)) return st;
   }
-  CK(cudaMemcpyAsync((char*)d->f + subs * bytes, f_host, bytes, cudaMemcpyHostToDevice,
-                     d->stream));
+  CK(lbx_internal_copy_in(d->p.device, d->stream, (char*)d->f + subs * bytes, f_host, bytes));
   if (lbx_status st = exchange(d, true)) return st;
   CK(cudaStreamSynchronize(d->stream));
   d->dense_stale = false;   // the compact state was just gathered from it
@@ -1039,8 +1040,7 @@ lbx_status lbx_download_f(lbx_domain* d, int subs, void* f_host)
   if (!f_host) return fail(LBX_ERR_INVALID, "f_host is NULL");
   const size_t bytes = (size_t)d->Q * d->N * d->real_size;
   if (d->dense_stale) { if (lbx_status st = exchange(d, false)) return st; }
-  CK(cudaMemcpyAsync(f_host, (char*)d->f + subs * bytes, bytes, cudaMemcpyDeviceToHost,
-                     d->stream));
+  CK(lbx_internal_copy_out(d->p.device, d->stream, f_host, (char*)d->f + subs * bytes, bytes));
   CK(cudaStreamSynchronize(d->stream));
   return LBX_OK;
 }
@@ -1050,8 +1050,7 @@ lbx_status lbx_upload_mv(lbx_domain* d, int subs, const void* mv_host)
   if (lbx_status st = check_subs(d, subs)) return st;
   if (!mv_host) return fail(LBX_ERR_INVALID, "mv_host is NULL");
   const size_t bytes = (size_t)(1 + d->D) * d->N * d->real_size;
-  CK(cudaMemcpyAsync((char*)d->mv + subs * bytes, mv_host, bytes, cudaMemcpyHostToDevice,
-                     d->stream));
+  CK(lbx_internal_copy_in(d->p.device, d->stream, (char*)d->mv + subs * bytes, mv_host, bytes));
   CK(cudaStreamSynchronize(d->stream));
   return LBX_OK;
 }
@@ -1062,9 +1061,13 @@ lbx_status lbx_download_mv(lbx_domain* d, int subs, void* rho, void* ux, void* u
   const size_t plane = (size_t)d->N * d->real_size;
   char* base = (char*)d->mv + (size_t)subs * (1 + d->D) * plane;
   void* dst[4] = {rho, ux, uy, uz};
-  for (int c = 0; c <= d->D; ++c)
-    if (dst[c])
-      CK(cudaMemcpyAsync(dst[c], base + c * plane, plane, cudaMemcpyDeviceToHost, d->stream));
+  for (int c = 0; c <= d->D;) {
+    // planes that lie behind one another on the host too are one copy
+    int n = 1;
+    while (dst[c] && c + n <= d->D && (char*)dst[c + n] == (char*)dst[c] + n * plane) ++n;
+    if (dst[c]) CK(lbx_internal_copy_out(d->p.device, d->stream, dst[c], base + c * plane, n * plane));
+    c += n;
+  }
   CK(cudaStreamSynchronize(d->stream));
   return LBX_OK;
 }
@@ -1090,7 +1093,7 @@ lbx_status lbx_init_equilibrium(lbx_domain* d, int subs, const void* rho, const 
   const void* src[4] = {rho, ux, uy, uz};
   cudaError_t e = cudaSuccess;
   for (int c = 0; c <= d->D && e == cudaSuccess; ++c)
-    e = src[c] ? cudaMemcpyAsync(t + c * plane, src[c], plane, cudaMemcpyHostToDevice, d->stream)
+    e = src[c] ? lbx_internal_copy_in(d->p.device, d->stream, t + c * plane, src[c], plane)
                : cudaMemsetAsync(t + c * plane, 0, plane, d->stream);
   if (e == cudaSuccess) {
     const int shifted = d->p.accurate && subs == 0;

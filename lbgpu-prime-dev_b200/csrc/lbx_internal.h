@@ -96,6 +96,15 @@ LBX_HIDDEN lbx_status lbx_internal_step_into(lbx_domain* d, int t, void* src, vo
 LBX_HIDDEN void lbx_internal_adjoint_free(lbx_domain* d);
 LBX_HIDDEN void lbx_internal_frames_free(lbx_domain* d);
 LBX_HIDDEN void lbx_internal_drop_graphs(lbx_domain* d);
+// Copies between device memory and the caller's host buffers, ordered after
+// the stream's earlier work (lbx_copy.cu): staged through page-locked chunks
+// and waited for where that is faster, else queued on the stream.  Each
+// domain registers as a user (add = 1, -1) of its device's chunks.
+LBX_HIDDEN cudaError_t lbx_internal_copy_out(int device, cudaStream_t stream, void* dst,
+                                             const void* src, size_t bytes);
+LBX_HIDDEN cudaError_t lbx_internal_copy_in(int device, cudaStream_t stream, void* dst,
+                                            const void* src, size_t bytes);
+LBX_HIDDEN void lbx_internal_copy_user(int device, int add);
 // PEST sampling: whether a sample is due at time t (the step then writes
 // the macro variables), the gather after that step, and the release.
 LBX_HIDDEN bool lbx_internal_pest_due(const lbx_domain* d, int t);
