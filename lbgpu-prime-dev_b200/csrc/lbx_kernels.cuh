@@ -230,7 +230,7 @@ __device__ __forceinline__ T signed_sum(S sign, const T (&v)[N])
 
 // c_a . u, its terms added in the order x, y, z.
 template <int D, typename T>
-__device__ __forceinline__ T cdotu(int a, const T (&u)[3])
+__device__ __forceinline__ T c_dot_u(int a, const T (&u)[3])
 {
   return signed_sum<3>([a](int q) { return q == 0 ? cx(a) : (q == 1 ? cy(a) : (D == 3 ? cz(a) : 0)); },
                        u);
@@ -255,9 +255,14 @@ __device__ __forceinline__ float collide_pairs(const StepArgs<float>& A, int s, 
     if (sinks == 2) rho *= A.sink1;
     rho *= A.sink1;
   } else {
-    const float m0 = signed_sum<NP>([](int p) { return cx(2 * p + 1); }, dif);
-    const float m1 = signed_sum<NP>([](int p) { return cy(2 * p + 1); }, dif);
-    const float m2 = D == 3 ? signed_sum<NP>([](int p) { return cz(2 * p + 1); }, dif) : 0.f;
+    float m0 = 0.f, m1 = 0.f, m2 = 0.f;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const int a = 2 * p + 1;
+      if (cx(a) > 0) m0 += dif[p]; else if (cx(a) < 0) m0 -= dif[p];
+      if (cy(a) > 0) m1 += dif[p]; else if (cy(a) < 0) m1 -= dif[p];
+      if (D == 3) { if (cz(a) > 0) m2 += dif[p]; else if (cz(a) < 0) m2 -= dif[p]; }
+    }
     const float den = (MODEL == SHIFTED_INC) ? c.rhoA
                     : (MODEL == PLAIN_COMP) ? rho : (c.rhoA + rho);
     const float inv = 1.f / den;
@@ -272,6 +277,13 @@ __device__ __forceinline__ float collide_pairs(const StepArgs<float>& A, int s, 
     m[2 * A.N + n] = u[1];
     if (D == 3) m[3 * A.N + n] = u[2];
   }
+  auto cdotu = [&](int a) -> float {
+    float r = 0.f;
+    if (cx(a) > 0) r += u[0]; else if (cx(a) < 0) r -= u[0];
+    if (cy(a) > 0) r += u[1]; else if (cy(a) < 0) r -= u[1];
+    if (D == 3) { if (cz(a) > 0) r += u[2]; else if (cz(a) < 0) r -= u[2]; }
+    return r;
+  };
   if (solute) {
     const float ci = rho * c.itau;
     d[0] = fmaf(d[0], c.omc, wgt<float, Q>(0) * ci);
@@ -279,7 +291,7 @@ __device__ __forceinline__ float collide_pairs(const StepArgs<float>& A, int s, 
     for (int p = 0; p < NP; ++p) {
       const int a = 2 * p + 1;
       const float base = wgt<float, Q>(a) * ci;
-      const float anti = (3.f * base) * cdotu<D>(a, u);
+      const float anti = (3.f * base) * cdotu(a);
       d[a] = fmaf(d[a], c.omc, base + anti);
       d[a + 1] = fmaf(d[a + 1], c.omc, base - anti);
     }
@@ -293,7 +305,7 @@ __device__ __forceinline__ float collide_pairs(const StepArgs<float>& A, int s, 
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       const int a = 2 * p + 1;
-      const float cu = cdotu<D>(a, u);
+      const float cu = cdotu(a);
       const float wq = wgt<float, Q>(a) * qi;
       const float sym = fmaf(wq, fmaf(4.5f * cu, cu, k), wgt<float, Q>(a) * ri);
       const float anti = (3.f * wq) * cu;
@@ -304,14 +316,16 @@ __device__ __forceinline__ float collide_pairs(const StepArgs<float>& A, int s, 
   return rho;
 }
 
-// The reference's operation order (FP64, Kahan sums and Walsh runs).  A pair
-// of opposite directions shares what its two equilibria compute alike: c.u
-// and 3 c.u change sign exactly, 4.5 (c.u)^2 does not change, and c.u is the
+// The reference's operation order (FP64, Kahan sums and Walsh runs).  In
+// FP64 a pair of opposite directions shares what its two equilibria compute
+// alike: c.u and 3 c.u change sign exactly, 4.5 (c.u)^2 does not change, and c.u is the
 // sum of its non-zero terms (products by 0 and 1 and sums with 0 change no
 // finite value), a quarter fewer FP64 operations, each rounded as before.
 // At 512 threads an SM's FP64 pipe bounds D2Q9's collision: 1416 cycles, 1634
 // with every direction on its own.
-// The momentum is divided by rho_A only where that is not 1 (m / 1 == m).
+// The FP64 momentum is divided by rho_A only where that is not 1 (m / 1 == m).
+// FP32 keeps the form of one direction at a time: the compiler's choice of
+// FMAs, and with it the results' last bits, goes with the form.
 template <typename T, int Q, int MODEL, bool WALSH = false>
 __device__ __forceinline__ T collide(const StepArgs<T>& A, int s, bool solute,
                                         int sinks, T (&d)[Q], T (&u)[3],
@@ -351,9 +365,19 @@ __device__ __forceinline__ T collide(const StepArgs<T>& A, int s, bool solute,
     if (sinks == 2) rho *= A.sink1;
     rho *= A.sink1;
   } else {
-    T m0 = signed_sum<Q>([](int a) { return cx(a); }, d);
-    T m1 = signed_sum<Q>([](int a) { return cy(a); }, d);
-    T m2 = D == 3 ? signed_sum<Q>([](int a) { return cz(a); }, d) : T(0);
+    T m0 = T(0), m1 = T(0), m2 = T(0);
+    if constexpr (sizeof(T) == 8) {
+      m0 = signed_sum<Q>([](int a) { return cx(a); }, d);
+      m1 = signed_sum<Q>([](int a) { return cy(a); }, d);
+      if (D == 3) m2 = signed_sum<Q>([](int a) { return cz(a); }, d);
+    } else {
+#pragma unroll
+      for (int a = 0; a < Q; ++a) {
+        if (cx(a) > 0) m0 += d[a]; else if (cx(a) < 0) m0 -= d[a];
+        if (cy(a) > 0) m1 += d[a]; else if (cy(a) < 0) m1 -= d[a];
+        if (D == 3) { if (cz(a) > 0) m2 += d[a]; else if (cz(a) < 0) m2 -= d[a]; }
+      }
+    }
     const T den = (MODEL == SHIFTED_INC) ? c.rhoA
                 : (MODEL == PLAIN_COMP) ? rho : (c.rhoA + rho);
     if (WALSH) {
@@ -366,15 +390,14 @@ __device__ __forceinline__ T collide(const StepArgs<T>& A, int s, bool solute,
       u[1] = (T)__dadd_rn((double)(m1 / den), __dmul_rn(ot, A.wg[s * 3 + 1]));
       u[2] = (D == 3) ? (T)__dadd_rn((double)(m2 / den), __dmul_rn(ot, A.wg[s * 3 + 2]))
                       : T(0);
-    } else {
-      if (MODEL != SHIFTED_INC || den != T(1)) {
-        m0 = m0 / den;
-        m1 = m1 / den;
-        if (D == 3) m2 = m2 / den;
-      }
+    } else if (sizeof(T) == 8 && MODEL == SHIFTED_INC && den == T(1)) {
       u[0] = add_(m0, c.tg[0]);
       u[1] = add_(m1, c.tg[1]);
       u[2] = (D == 3) ? add_(m2, c.tg[2]) : T(0);
+    } else {
+      u[0] = add_(m0 / den, c.tg[0]);
+      u[1] = add_(m1 / den, c.tg[1]);
+      u[2] = (D == 3) ? add_(m2 / den, c.tg[2]) : T(0);
     }
   }
   if (write_mv) {
@@ -386,19 +409,27 @@ __device__ __forceinline__ T collide(const StepArgs<T>& A, int s, bool solute,
   }
   if (solute) {
     // g_a <- g_a (1 - 1/tau_s) + w_a C (1 + 3 c.u) / tau_s  (src/lattice.c:2858-2875)
-    d[0] = add_(mul_(d[0], c.omc), mul_(mul_(wgt<T, Q>(0), rho), c.itau));
+    if constexpr (sizeof(T) == 8) {
+      d[0] = add_(mul_(d[0], c.omc), mul_(mul_(wgt<T, Q>(0), rho), c.itau));
 #pragma unroll
-    for (int a = 1; a < Q; a += 2) {
-      const T wr = mul_(wgt<T, Q>(a), rho), cu3 = mul_(T(3), cdotu<D>(a, u));
-      d[a] = add_(mul_(d[a], c.omc), mul_(mul_(wr, add_(T(1), cu3)), c.itau));
-      d[a + 1] = add_(mul_(d[a + 1], c.omc), mul_(mul_(wr, sub_(T(1), cu3)), c.itau));
+      for (int a = 1; a < Q; a += 2) {
+        const T wr = mul_(wgt<T, Q>(a), rho), cu3 = mul_(T(3), c_dot_u<D>(a, u));
+        d[a] = add_(mul_(d[a], c.omc), mul_(mul_(wr, add_(T(1), cu3)), c.itau));
+        d[a + 1] = add_(mul_(d[a + 1], c.omc), mul_(mul_(wr, sub_(T(1), cu3)), c.itau));
+      }
+    } else {
+#pragma unroll
+      for (int a = 0; a < Q; ++a) {
+        T cu = T(cx(a)) * u[0] + T(cy(a)) * u[1] + (D == 3 ? T(cz(a)) * u[2] : T(0));
+        d[a] = add_(mul_(d[a], c.omc),
+                    mul_(mul_(mul_(wgt<T, Q>(a), rho), add_(T(1), mul_(T(3), cu))), c.itau));
+      }
     }
   } else {
     // BGK in shifted or plain form (src/lattice.c:2880-2919):
     // d (1 - 1/tau) + w drho / tau + w rq (3 cu + 4.5 cu^2 - 1.5 u^2) / tau
     T usq = add_(mul_(u[0], u[0]), mul_(u[1], u[1]));
     if (D == 3) usq = add_(usq, mul_(u[2], u[2]));
-    const T u15 = mul_(T(1.5), usq);
     const T rq = (MODEL == SHIFTED_INC) ? c.rhoA
                : (MODEL == PLAIN_COMP) ? rho : (c.rhoA + rho);
     auto relax = [&](int a, T poly) {
@@ -406,13 +437,23 @@ __device__ __forceinline__ T collide(const StepArgs<T>& A, int s, bool solute,
       d[a] = add_(add_(mul_(d[a], c.omc), mul_(mul_(w, rho), c.itau)),
                   mul_(mul_(mul_(w, rq), poly), c.itau));
     };
-    relax(0, -u15);
+    if constexpr (sizeof(T) == 8) {
+      const T u15 = mul_(T(1.5), usq);
+      relax(0, -u15);
 #pragma unroll
-    for (int a = 1; a < Q; a += 2) {
-      const T cu = cdotu<D>(a, u);
-      const T cu3 = mul_(T(3), cu), cu45 = mul_(mul_(T(4.5), cu), cu);
-      relax(a, sub_(add_(cu3, cu45), u15));
-      relax(a + 1, sub_(sub_(cu45, cu3), u15));
+      for (int a = 1; a < Q; a += 2) {
+        const T cu = c_dot_u<D>(a, u);
+        const T cu3 = mul_(T(3), cu), cu45 = mul_(mul_(T(4.5), cu), cu);
+        relax(a, sub_(add_(cu3, cu45), u15));
+        relax(a + 1, sub_(sub_(cu45, cu3), u15));
+      }
+    } else {
+#pragma unroll
+      for (int a = 0; a < Q; ++a) {
+        // c.u: products by -1, 0, 1 are exact, so contraction cannot change it
+        T cu = T(cx(a)) * u[0] + T(cy(a)) * u[1] + (D == 3 ? T(cz(a)) * u[2] : T(0));
+        relax(a, sub_(add_(mul_(T(3), cu), mul_(mul_(T(4.5), cu), cu)), mul_(T(1.5), usq)));
+      }
     }
   }
   if (WALSH) {
