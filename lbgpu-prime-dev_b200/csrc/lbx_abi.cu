@@ -251,7 +251,7 @@ void launch_nodes(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fuse
     auto go = [&](auto odd_c, auto idx_c, auto oop_c) {
       constexpr bool o = decltype(odd_c)::value;
       if constexpr (step_joint<Q, NS, o, true>() == (PART == PART_ALL)) {
-        constexpr int bs = compact_threads<T, NS, o, PART, false>();
+        const unsigned bs = compact_block<T, NS, o, PART, false>(count);
         aa_step_compact<T, Q, NS, MODEL, o, PART, decltype(idx_c)::value, decltype(oop_c)::value>
             <<<((unsigned)count + bs - 1) / bs, bs, 0, d->stream>>>(C);
       }

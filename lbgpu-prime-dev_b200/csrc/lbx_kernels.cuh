@@ -723,28 +723,41 @@ struct CompactArgs {
   int m_base, m_skip, m_jump, m_end;
 };
 
-// Threads per block and resident blocks asked of the compiler, compact
-// kernels (microseconds of one launch, 256^3 at porosity 0.4 unless said
-// otherwise).  FP32: odd flow six blocks of 256 threads (40 registers; 213,
-// five 222), even four (flow 165 at six, 162 at four; 192 x 192 x 384 at
-// porosity 0.35, flow then solute: 128 + 129 at six, 126 + 125 at four).
-// FP64: odd flow six of 128 (80 registers: 256-thread blocks leave an eighth
-// of the register file idle; 391 -> 375), even three of 256 (307).  Two
-// substances in one thread: odd FP32 192 x 192 x 384 four of 256 (64
-// registers, 313), odd FP64 192^3 four of 128 (346 -> 332); D2Q9 likewise.
-// The z-face planes' nodes (FACES3) are few and their rules need registers:
-// four of 128.
+// Threads per block (at most, for the even kernels: see compact_block) and
+// resident blocks asked of the compiler, compact kernels (microseconds of one
+// launch, 256^3 at porosity 0.4 unless said otherwise).  FP32: odd flow
+// twelve blocks of 128 threads (40 registers; 213, ten 227), even 64
+// registers (flow 165 at 40, 162 at 64; 192 x 192 x 384 at porosity 0.35,
+// flow then solute: 128 + 129, 126 + 125).  FP64: odd flow six of 128 (80
+// registers: 256-thread blocks leave an eighth of the register file idle;
+// 391 -> 375), even 80 registers (307).  Two substances in one thread: odd
+// FP32 192 x 192 x 384 four of 256 (64 registers, 313), odd FP64 192^3 four
+// of 128 (346 -> 332); D2Q9 likewise.  The z-face planes' nodes (FACES3) are
+// few and their rules need registers: four of 128.
 template <typename T, int NS, bool ODD, int PART, bool FACES3>
 __host__ __device__ constexpr int compact_threads()
 {
-  return FACES3 || (sizeof(T) == 8 && (ODD || (NS == 2 && PART == PART_ALL))) ? 128 : 256;
+  if (NS == 2 && PART == PART_ALL && !FACES3) return sizeof(T) == 8 ? 128 : 256;
+  return FACES3 || ODD ? 128 : 256;
 }
 
 template <typename T, int NS, bool ODD, int PART, bool FACES3>
 __host__ __device__ constexpr int compact_min_blocks()
 {
-  if (FACES3 || (NS == 2 && PART == PART_ALL)) return 4;
-  return sizeof(T) == 4 ? (ODD ? 6 : 4) : (ODD ? 6 : 3);
+  if (FACES3) return 4;
+  if (NS == 2 && PART == PART_ALL) return 4;
+  return sizeof(T) == 4 ? (ODD ? 12 : 4) : (ODD ? 6 : 3);
+}
+
+// The threads per block of a launch over `count` nodes: blocks of 128 spread
+// evenly over the SMs where there are only a few per SM (FP32 step pair at
+// 64^3, porosity 0.5: 10.4 us with 256-thread blocks, 9.4 with 128; 96^3
+// 23.6 and 22.5), 256 stream a little faster where there are many (even step
+// at 256^3 162 against 163; equal at a million nodes).
+template <typename T, int NS, bool ODD, int PART, bool FACES3>
+constexpr int compact_block(long long count)
+{
+  return count < (1 << 20) ? 128 : compact_threads<T, NS, ODD, PART, FACES3>();
 }
 
 // IDX32: population offsets within one substance's [Q][P] block fit in 32
