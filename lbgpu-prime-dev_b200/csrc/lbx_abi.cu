@@ -771,7 +771,14 @@ lbx_status capture_pairs(lbx_domain* d, int t, int npairs, cudaGraphExec_t* out,
 // `pairs` AA pairs with the launch arguments of the pair at t, replayed from
 // graphs of one pair and of kGraphPairs pairs (fewer graph launches, and
 // the kernels of a multi-pair graph follow each other without the host).
+// A short stretch of long steps is launched directly: the launches run ahead
+// of the GPU, and capturing the graphs would hold it up (1-2 ms for a step
+// with z faces and a record, the GPU time of 30 such steps at 128 x 112 x
+// 96).  Populations of 50 MB (100 moved) step in some 20 us, more than the
+// launches of a step with faces take.
 constexpr int kGraphPairs = 8;
+constexpr int kDirectPairs = 64;
+constexpr double kDirectBytes = 50e6;
 
 lbx_status replay_pairs(lbx_domain* d, int t, int pairs)
 {
@@ -782,6 +789,13 @@ lbx_status replay_pairs(lbx_domain* d, int t, int pairs)
   const size_t klen = k1 + k2;
   if (!d->graph || d->graph_stream != d->stream || d->graph_key_len != klen ||
       std::memcmp(d->graph_key, key, klen) != 0) {
+    const double bytes = (double)d->p.nsubs * d->Q * (double)d->real_size *
+                         (double)(d->layout == LBX_LAYOUT_COMPACT ? d->fluid : d->N);
+    if (pairs < kDirectPairs && bytes > kDirectBytes) {
+      for (int q = 0; q < 2 * pairs; ++q)
+        if (lbx_status st = do_step(d, t + q, 0)) return st;
+      return LBX_OK;
+    }
     // both graphs at once, so a later, longer stretch does not pay a capture
     lbx_internal_drop_graphs(d);
     if (lbx_status st = capture_pairs(d, t, 1, &d->graph, &d->graph_launches)) return st;
@@ -834,23 +848,25 @@ lbx_status tiled_pairs(lbx_domain* d, int t, int pairs, bool write_mv)
   return st;
 }
 
-// Dense exchange array <-> compact populations.
-lbx_status exchange(lbx_domain* d, bool to_compact)
+// Dense exchange array <-> compact populations, of one substance or (-1) all.
+lbx_status exchange(lbx_domain* d, bool to_compact, int subs = -1)
 {
   if (d->layout != LBX_LAYOUT_COMPACT || d->fluid == 0) return LBX_OK;
-  const int planes = d->p.nsubs * d->Q;
+  const int planes = (subs < 0 ? d->p.nsubs : 1) * d->Q;
+  const int first = subs < 0 ? 0 : subs * d->Q;
   const long long total = d->fluid * planes;
   const unsigned blocks = (unsigned)((total + 255) / 256);
-  if (d->real_size == 8) {
-    if (to_compact) gather_compact<double><<<blocks, 256, 0, d->stream>>>((double*)d->fc, (const double*)d->f, d->fnode, (int)d->fluid, (int)d->P, d->N, planes);
-    else scatter_compact<double><<<blocks, 256, 0, d->stream>>>((double*)d->f, (const double*)d->fc, d->fnode, (int)d->fluid, (int)d->P, d->N, planes);
-  } else {
-    if (to_compact) gather_compact<float><<<blocks, 256, 0, d->stream>>>((float*)d->fc, (const float*)d->f, d->fnode, (int)d->fluid, (int)d->P, d->N, planes);
-    else scatter_compact<float><<<blocks, 256, 0, d->stream>>>((float*)d->f, (const float*)d->fc, d->fnode, (int)d->fluid, (int)d->P, d->N, planes);
-  }
+  auto go = [&](auto real) {
+    using T = decltype(real);
+    T* const fc = (T*)d->fc + (size_t)first * d->P;
+    T* const f = (T*)d->f + (size_t)first * d->N;
+    if (to_compact) gather_compact<T><<<blocks, 256, 0, d->stream>>>(fc, f, d->fnode, (int)d->fluid, (int)d->P, d->N, planes);
+    else scatter_compact<T><<<blocks, 256, 0, d->stream>>>(f, fc, d->fnode, (int)d->fluid, (int)d->P, d->N, planes);
+  };
+  if (d->real_size == 8) go(double()); else go(float());
   d->launches++;
   CK(cudaGetLastError());
-  if (!to_compact) d->dense_stale = false;
+  if (!to_compact && subs < 0) d->dense_stale = false;
   return LBX_OK;
 }
 
@@ -1020,16 +1036,12 @@ lbx_status lbx_upload_f(lbx_domain* d, int subs, const void* f_host)
   if (lbx_status st = check_subs(d, subs)) return st;
   if (!f_host) return fail(LBX_ERR_INVALID, "f_host is NULL");
   const size_t bytes = (size_t)d->Q * d->N * d->real_size;
-  // the other substance's dense copy must be current before the gather; a
-  // single substance is overwritten whole, so its stale copy is not brought
-  // back first
-  if (d->dense_stale && d->p.nsubs > 1) {
-    if (lbx_status st = exchange(d, false)) return st;
-  }
+  // this substance is overwritten whole and gathered alone; another one's
+  // stale dense copy stays behind its compact state
   CK(lbx_internal_copy_in(d->p.device, d->stream, (char*)d->f + subs * bytes, f_host, bytes));
-  if (lbx_status st = exchange(d, true)) return st;
+  if (lbx_status st = exchange(d, true, subs)) return st;
   CK(cudaStreamSynchronize(d->stream));
-  d->dense_stale = false;   // the compact state was just gathered from it
+  if (d->p.nsubs == 1) d->dense_stale = false;   // the compact state was gathered from it
   d->parity = 0;
   return LBX_OK;
 }
@@ -1077,12 +1089,6 @@ lbx_status lbx_init_equilibrium(lbx_domain* d, int subs, const void* rho, const 
 {
   if (lbx_status st = check_subs(d, subs)) return st;
   if (!rho) return fail(LBX_ERR_INVALID, "rho is required");
-  // as in lbx_upload_f: the other substance's dense copy must be current
-  // before the gather; a single substance is overwritten whole, so its
-  // stale copy is not brought back first
-  if (d->dense_stale && d->p.nsubs > 1) {
-    if (lbx_status st = exchange(d, false)) return st;
-  }
   // the fields land in the substance's macro variables, where the
   // reference's init_problem leaves them (src/latman.c:1302-1780), and the
   // populations are formed from there: no staging allocation.  A velocity
@@ -1113,11 +1119,11 @@ lbx_status lbx_init_equilibrium(lbx_domain* d, int subs, const void* rho, const 
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && d->layout == LBX_LAYOUT_COMPACT) {
-    if (exchange(d, true) != LBX_OK) e = cudaErrorUnknown;
+    if (exchange(d, true, subs) != LBX_OK) e = cudaErrorUnknown;   // as in lbx_upload_f
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(d->stream);
   if (e != cudaSuccess) return fail(LBX_ERR_CUDA, "init_equilibrium: %s", cudaGetErrorString(e));
-  d->dense_stale = false;   // the compact state was just gathered from it
+  if (d->p.nsubs == 1) d->dense_stale = false;   // the compact state was gathered from it
   d->parity = 0;
   return LBX_OK;
 }

@@ -777,6 +777,7 @@ lbx_status lbx_batch_create(int nsamples, const lbx_params* params, const uint8_
   BCKD(cudaMemset(b->mv, 0, (size_t)(1 + b->dims) * b->Ntot * rs));
   if (lbx_status st = lay_out(b, LBX_BATCH_LAYOUT_LARGEST_FIRST, sol)) return bail(st);
 #undef BCKD
+  lbx_internal_copy_user(b->device, 1);
   *out = b;
   return LBX_OK;
 }
@@ -786,6 +787,7 @@ lbx_status lbx_batch_destroy(lbx_batch* b)
   if (!b) return LBX_OK;
   if (b->stream) cudaStreamSynchronize(b->stream);
   release(b);
+  lbx_internal_copy_user(b->device, -1);
   delete b;
   return LBX_OK;
 }
@@ -796,8 +798,9 @@ lbx_status lbx_batch_upload_f(lbx_batch* b, int s, const void* f_host)
   if (!f_host) return bfail(LBX_ERR_INVALID, "f_host is NULL");
   if (lbx_status st = sync_dense(b)) return st;
   const size_t rs = (size_t)b->precision;
-  BCK(cudaMemcpyAsync((char*)b->fdense + (size_t)b->fbase_dense[s] * rs, f_host,
-                      (size_t)b->Q * b->N[s] * rs, cudaMemcpyHostToDevice, b->stream));
+  BCK(lbx_internal_copy_in(b->device, b->stream,
+                           (char*)b->fdense + (size_t)b->fbase_dense[s] * rs, f_host,
+                           (size_t)b->Q * b->N[s] * rs));
   if (lbx_status st = exchange(b, s, true)) return st;
   BCK(cudaStreamSynchronize(b->stream));
   b->parity = 0;
@@ -810,8 +813,9 @@ lbx_status lbx_batch_download_f(lbx_batch* b, int s, void* f_host)
   if (!f_host) return bfail(LBX_ERR_INVALID, "f_host is NULL");
   if (lbx_status st = sync_dense(b)) return st;
   const size_t rs = (size_t)b->precision;
-  BCK(cudaMemcpyAsync(f_host, (char*)b->fdense + (size_t)b->fbase_dense[s] * rs,
-                      (size_t)b->Q * b->N[s] * rs, cudaMemcpyDeviceToHost, b->stream));
+  BCK(lbx_internal_copy_out(b->device, b->stream, f_host,
+                            (char*)b->fdense + (size_t)b->fbase_dense[s] * rs,
+                            (size_t)b->Q * b->N[s] * rs));
   BCK(cudaStreamSynchronize(b->stream));
   return LBX_OK;
 }
@@ -867,7 +871,7 @@ lbx_status lbx_batch_download_mv(lbx_batch* b, int s, void* rho, void* ux, void*
     int n = 1;
     while (dst[c] && c + n <= b->dims && (char*)dst[c + n] == (char*)dst[c] + n * plane) ++n;
     if (dst[c])
-      BCK(cudaMemcpyAsync(dst[c], base + c * plane, n * plane, cudaMemcpyDeviceToHost, b->stream));
+      BCK(lbx_internal_copy_out(b->device, b->stream, dst[c], base + c * plane, n * plane));
     c += n;
   }
   BCK(cudaStreamSynchronize(b->stream));

@@ -4,14 +4,15 @@
 // A plain copy into a freshly allocated pageable buffer runs at 5 GB/s here:
 // the driver stages it on one thread, which also takes the buffer's page
 // faults (the four macro-variable planes of 150 x 131 x 117 FP64 nodes, 74
-// MB, took 14.6 ms of a 29 ms job).  Copies of 16 MB or more go through
-// page-locked chunks instead, filled or emptied by several host threads
-// while the next chunks cross the link.  Smaller copies, buffers the caller
-// has page-locked, and any failure to set this up take the plain copy.
+// MB, took 14.6 ms of a 29 ms job; 2.4 ms staged).  Copies of 4 MB or more go
+// through page-locked chunks instead, filled or emptied by several host
+// threads while the next chunks cross the link; a smaller one is done about
+// when the threads have started (0.1 ms).  Smaller copies, buffers the
+// caller has page-locked, and any failure to set this up take the plain copy.
 //
 // The chunks (one set per device, 1 MB x 2 x threads, at most 16 MB) live
-// while any domain of the device does: made by the first large copy, given
-// back when the last domain is destroyed.  One copy uses them at a time; a
+// while any domain or batch of the device does: made by the first large copy,
+// given back when the last is destroyed.  One copy uses them at a time; a
 // copy that finds them taken by another host thread is a plain one.
 #include "lbx.h"
 #include "lbx_internal.h"
@@ -26,7 +27,7 @@
 namespace {
 
 constexpr size_t kChunk = 1 << 20;
-constexpr size_t kStaged = 16 << 20;    // copies from this size on are staged
+constexpr size_t kStaged = 4 << 20;     // copies from this size on are staged
 constexpr int kMaxWorkers = 8;
 
 struct Worker {
@@ -196,7 +197,7 @@ void lbx_internal_copy_user(int device, int add)
     Stage& s = g_stages[device];
     s.users += add;
     if (s.users > 0) return;
-    // no domain is left on the device, so no copy is under way
+    // no domain or batch is left on the device, so no copy is under way
     tear_down(s);
     s.failed = false;
   } catch (...) {}

@@ -99,7 +99,7 @@ LBX_HIDDEN void lbx_internal_drop_graphs(lbx_domain* d);
 // Copies between device memory and the caller's host buffers, ordered after
 // the stream's earlier work (lbx_copy.cu): staged through page-locked chunks
 // and waited for where that is faster, else queued on the stream.  Each
-// domain registers as a user (add = 1, -1) of its device's chunks.
+// domain and batch registers as a user (add = 1, -1) of its device's chunks.
 LBX_HIDDEN cudaError_t lbx_internal_copy_out(int device, cudaStream_t stream, void* dst,
                                              const void* src, size_t bytes);
 LBX_HIDDEN cudaError_t lbx_internal_copy_in(int device, cudaStream_t stream, void* dst,

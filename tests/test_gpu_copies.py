@@ -19,8 +19,8 @@ def _domain(n):
     return lbx.Domain(p, np.zeros(n, np.uint8))
 
 
-# bytes of [19][n] floats: below, at and above 16 MB, one with a ragged last chunk
-@pytest.mark.parametrize("n", [16 * MB // 76 - 3, 16 * MB // 76 + 1, 16 * MB // 76 + 13797 * 3 + 1,
+# bytes of [19][n] floats: below, at and above 4 MB, one with a ragged last chunk
+@pytest.mark.parametrize("n", [4 * MB // 76 - 3, 4 * MB // 76 + 1, 4 * MB // 76 + 13797 * 3 + 1,
                                500_001])
 def test_populations_round_trip(n):
     f = np.random.default_rng(n).random((1, 19, n)).astype(np.float32)
@@ -60,3 +60,16 @@ def test_threads_and_reuse():
         [t.start() for t in ts]
         [t.join() for t in ts]
         assert all(np.array_equal(o, f) for o, f in zip(out, fs))
+
+
+def test_batch_samples():
+    from lbx.batch import Batch
+    edges = [40, 97]
+    ps = [lbx.Params(dims=3, LX=e, LY=e, LZ=e, precision=4) for e in edges]
+    rng = np.random.default_rng(2)
+    ms = [(rng.random(p.NN) < 0.3).astype(np.uint8) for p in ps]
+    with Batch(ps, ms) as b:
+        fs = [rng.random((19, p.NN)).astype(np.float32) for p in ps]
+        for i, f in enumerate(fs):
+            b.upload_f(i, f)
+        assert all(np.array_equal(b.download_f(i), f) for i, f in enumerate(fs))
