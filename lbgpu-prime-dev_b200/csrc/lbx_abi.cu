@@ -232,6 +232,25 @@ void launch_face_nodes(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face
   }
 }
 
+// A step kernel's launch; dependent: as a programmatic dependent of the
+// kernel before it in the stream (see pdl_wait).
+template <typename... P, typename... A>
+void launch_step_kernel(void (*kernel)(P...), unsigned blocks, unsigned threads,
+                        cudaStream_t stream, bool dependent, const A&... args)
+{
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = dependent ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, args...);   // a failure stays for cudaGetLastError
+}
+
 // One launch over the lattice (compact: over the interior between the
 // z-face planes when f3 is given; launch_face_nodes takes the two planes).
 template <typename T, int Q, int NS, int MODEL, int PART>
@@ -239,6 +258,9 @@ void launch_nodes(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fuse
 {
   using TT = std::true_type;
   using FF = std::false_type;
+  // Steps whose kernels follow one another in the stream do so closely; with
+  // a second stream, a record or stored states beside them they stay plain.
+  const bool dependent = !d->btc_vals && !A.fout && !d->faces3_active;
   if (d->layout == LBX_LAYOUT_COMPACT) {
     CompactArgs<T> C = make_compact<T>(d, A);
     if (f3) {
@@ -252,8 +274,9 @@ void launch_nodes(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fuse
       constexpr bool o = decltype(odd_c)::value;
       if constexpr (step_joint<Q, NS, o, true>() == (PART == PART_ALL)) {
         const unsigned bs = compact_block<T, NS, o, PART, false>(count);
-        aa_step_compact<T, Q, NS, MODEL, o, PART, decltype(idx_c)::value, decltype(oop_c)::value>
-            <<<((unsigned)count + bs - 1) / bs, bs, 0, d->stream>>>(C);
+        launch_step_kernel(aa_step_compact<T, Q, NS, MODEL, o, PART, decltype(idx_c)::value,
+                                           decltype(oop_c)::value>,
+                           ((unsigned)count + bs - 1) / bs, bs, d->stream, dependent, C);
       }
     };
     if (A.fout) {
@@ -271,8 +294,9 @@ void launch_nodes(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fuse
   auto go = [&](auto odd_c, auto idx_c, auto walsh_c) {
     constexpr bool o = decltype(odd_c)::value;
     if constexpr (step_joint<Q, NS, o, false>() == (PART == PART_ALL))
-      aa_step<T, Q, NS, MODEL, o, PART, decltype(idx_c)::value, decltype(walsh_c)::value>
-          <<<(unsigned)((A.N + 255) / 256), 256, 0, d->stream>>>(A, dp, dl);
+      launch_step_kernel(aa_step<T, Q, NS, MODEL, o, PART, decltype(idx_c)::value,
+                                 decltype(walsh_c)::value>,
+                         (unsigned)((A.N + 255) / 256), 256, d->stream, dependent, A, dp, dl);
   };
   if (A.ns) {
     if (idx32) { if (odd) go(TT{}, TT{}, TT{}); else go(FF{}, TT{}, TT{}); }
