@@ -498,8 +498,11 @@ bool make_tiles(const FluidSums& fs, int LX, int LY, const Shape& sh, int cap,
       const int x = edge(c), w = edge(c + 1) - x;
       const int hmax = cap / tiled_pitch(w, K) - 2 * K;
       for (int y = 0; y < LY && n <= sh.tiles; ++n) {
-        int h = 1;
-        while (h < hmax && y + h < LY && fs.work(x, y, w, h + 1, K) <= W) ++h;
+        int h = 1, most = std::min(hmax, LY - y);     // the work grows with h
+        while (h < most) {
+          const int mid = (h + most + 1) / 2;
+          if (fs.work(x, y, w, mid, K) <= W) h = mid; else most = mid - 1;
+        }
         if (to) {
           Tile t;
           std::memset(&t, 0, sizeof t);
