@@ -1171,13 +1171,18 @@ lbx_status lbx_run(lbx_domain* d, int t0, int nsteps, int frame_rate)
   if (nsteps < 0) return fail(LBX_ERR_INVALID, "nsteps must be >= 0");
   const int tend = t0 + nsteps;
   int t = t0 + 1;
+  // Captured by the caller, every step is a launch of its own: a graph cannot
+  // be made or launched inside a capture, a plan's tables would be copied
+  // from host memory gone at the replay, and a tiled launch holds counters
+  // that a replay would find already reached.
+  const bool captured = lbx_internal_capturing(d->stream);
   alignas(16) unsigned char k_odd[kKey], k_even[kKey], k[kKey];
   while (t <= tend) {
     const bool frame = frame_rate > 0 && t % frame_rate == 0;
     // a stretch of steps starting on an odd time with the launch arguments
     // of its first pair throughout: of two or more frame-free pairs it is
     // replayed from a graph; the tiled run takes a frame's even step with it
-    if (!frame && (t % 2) == 1 && d->parity == 0 && tend - t + 1 >= 4) {
+    if (!captured && !frame && (t % 2) == 1 && d->parity == 0 && tend - t + 1 >= 4) {
       const size_t ko = step_key(d, t, k_odd), ke = step_key(d, t + 1, k_even);
       int pairs = 0;
       bool frame_last = false;    // the pair after the frame-free ones ends in a frame

@@ -178,7 +178,8 @@ bool staged(int device, cudaStream_t stream, void* dst, const void* src, size_t 
 
 cudaError_t copy(int device, cudaStream_t stream, void* dst, const void* src, size_t bytes, bool out)
 {
-  if (bytes >= kStaged && pageable(out ? dst : src)) {
+  // (in a caller's capture the event below would draw the workers' streams in)
+  if (bytes >= kStaged && pageable(out ? dst : src) && !lbx_internal_capturing(stream)) {
     try {
       cudaError_t e = cudaSuccess;
       if (staged(device, stream, dst, src, bytes, out, &e)) return e;
@@ -189,6 +190,17 @@ cudaError_t copy(int device, cudaStream_t stream, void* dst, const void* src, si
 }
 
 }  // namespace
+
+bool lbx_internal_capturing(cudaStream_t stream)
+{
+  if (!stream) return false;            // the default stream cannot be captured
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return status != cudaStreamCaptureStatusNone;
+}
 
 void lbx_internal_copy_user(int device, int add)
 {

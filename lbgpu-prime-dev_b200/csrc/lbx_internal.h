@@ -118,6 +118,8 @@ LBX_HIDDEN void lbx_internal_pest_free(lbx_domain* d);
 // Bytes the tiled run of this lattice would like behind the population
 // array (0: it would not be taken).
 LBX_HIDDEN size_t lbx_internal_tiled_room(const lbx_domain* d);
+// Whether the caller is capturing `stream` into a graph of its own.
+LBX_HIDDEN bool lbx_internal_capturing(cudaStream_t stream);
 LBX_HIDDEN lbx_status lbx_internal_tiled_plan(lbx_domain* d, bool* better);
 template <typename T>
 LBX_HIDDEN lbx_status lbx_internal_tiled_run(lbx_domain* d, const lbx::StepArgs<T>& A, int pairs,
