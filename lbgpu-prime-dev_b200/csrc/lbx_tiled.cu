@@ -444,12 +444,19 @@ double shape_us(double fluid, int w, int h, int K)
          lat;
 }
 
-// The launch-per-step path's: a launch and the populations, from the L2
-// (FP64 2.4 us for 2k fluid nodes, 2.9 for 39k, 3.7 for 104k, 5.7 for 227k;
-// 3.7 for 43k with a solute; FP32 2.5 for 39k, 4.1 for 170k).
+// The launch-per-step path's: a latency, larger for two substances (two
+// launches or a joint one), and the populations, from the L2.  Fitted to
+// whole runs of dependent launches, 40 % / 2 % solid nodes (modelled /
+// measured, us per step): FP64 256^2 2.4, 2.8 / 2.2, 2.5, 400^2 3.2, 4.2 /
+// 3.1, 4.3, 560^2 4.6, 6.4 / 4.9, 6.3; FP32 512^2 3.5, 4.6 / 3.7, 3.8; FP64
+// with a solute 200^2 2.9, 3.3 / 2.9, 3.4, 380^2 4.5, 6.0 / 4.7, 6.2.  With
+// the latency of launches that waited for one another (2.3 us, one
+// substance) the tiled run was taken where it lost: 560^2 FP64 5.5 against
+// 4.9, 380^2 with a solute 6.2 against 4.7.
 double steps_us(double nodes, size_t real, int nsubs)
 {
-  return 2.3 + nodes * nsubs * (real == 8 ? 1.5e-5 : 1.2e-5);
+  const double per = real != 8 ? 1.1e-5 : nsubs == 2 ? 1.3e-5 : 1.5e-5;
+  return (nsubs == 2 ? 2.3 : 1.8) + nodes * nsubs * per;
 }
 
 // The shapes whose regions fit a block and whose tiles fit the SMs: the best
