@@ -10,8 +10,9 @@
 // population array and a scratch copy of it, so a round never reads what a
 // slower block of the same round writes.  The rounds of one launch are even
 // in number (the state ends in the population array), of even length each
-// (a round ends after an even step), K steps or fewer: any number of AA
-// pairs from two on is one launch.
+// (a round ends after an even step), K steps or fewer (none in the first
+// round where K is 2 and the pairs are odd in number): any number of AA pairs
+// from two on is one launch.
 //
 // Between rounds a block waits only for the tiles its halo reads (their
 // round counters, polled by one lane each; the wait is bounded and records a
@@ -122,11 +123,37 @@ struct TiledArgs {
   int write_mv;                 // the last step writes the macro variables
 };
 
-// Steps of round r: the pairs spread evenly, the first rounds one longer.
-__device__ __forceinline__ int round_steps(int pairs, int rounds, int r)
+// Rounds of a stretch of `pairs` AA pairs at K steps a round at most: an even
+// number, two at least.  At K = 2 that is one more than the pairs where these
+// are odd, so one round has no step.
+__host__ __device__ constexpr int round_count(int pairs, int K)
 {
-  return 2 * (pairs / rounds + (r < pairs % rounds ? 1 : 0));
+  const int per = K / 2, least = ((pairs + per - 1) / per + 1) / 2 * 2;
+  return least < 2 ? 2 : least;
 }
+
+// Steps of round r: the pairs spread evenly, the last rounds one longer, so
+// that the last one always has the step that writes the macro variables.
+__host__ __device__ constexpr int round_steps(int pairs, int rounds, int r)
+{
+  return 2 * (pairs / rounds + (r >= rounds - pairs % rounds ? 1 : 0));
+}
+
+constexpr bool rounds_end_in_steps()
+{
+  for (int K = 2; K <= kMaxK; K += 2)
+    for (int pairs = 2; pairs <= 60; ++pairs) {
+      const int rounds = round_count(pairs, K);
+      int steps = 0;
+      for (int r = 0; r < rounds; ++r) {
+        if (round_steps(pairs, rounds, r) > K) return false;
+        steps += round_steps(pairs, rounds, r);
+      }
+      if (steps != 2 * pairs || round_steps(pairs, rounds, rounds - 1) < 2) return false;
+    }
+  return true;
+}
+static_assert(rounds_end_in_steps(), "every stretch's steps, the last round with some");
 
 // Round counters: tile t has stored the strips of round r when
 // flags[t] >= base + r + 1 (base grows from launch to launch).
@@ -688,9 +715,7 @@ lbx_status launch(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
   constexpr size_t smem = tiled_smem<T, NS>();
   const void* fn = (const void*)aa_tiled<T, NS, MODEL>;
   const int nt = d->tiled_ntiles;
-  // an even number of rounds of at most tiled_k steps, two at least
-  const int per = d->tiled_k / 2;
-  const int rounds = std::max(2, ((pairs + per - 1) / per + 1) / 2 * 2);
+  const int rounds = round_count(pairs, d->tiled_k);
   cudaError_t e = cudaSuccess;
   if (!d->tiled_attr) {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
