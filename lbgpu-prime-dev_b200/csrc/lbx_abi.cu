@@ -1182,7 +1182,9 @@ lbx_status lbx_run(lbx_domain* d, int t0, int nsteps, int frame_rate)
     // a stretch of steps starting on an odd time with the launch arguments
     // of its first pair throughout: of two or more frame-free pairs it is
     // replayed from a graph; the tiled run takes a frame's even step with it
-    if (!captured && !frame && (t % 2) == 1 && d->parity == 0 && tend - t + 1 >= 4) {
+    // (not on the CUDA default stream, which takes neither)
+    if (!captured && !frame && (t % 2) == 1 && d->parity == 0 && d->stream != nullptr &&
+        tend - t + 1 >= 4) {
       const size_t ko = step_key(d, t, k_odd), ke = step_key(d, t + 1, k_even);
       int pairs = 0;
       bool frame_last = false;    // the pair after the frame-free ones ends in a frame
@@ -1197,14 +1199,14 @@ lbx_status lbx_run(lbx_domain* d, int t0, int nsteps, int frame_rate)
       }
       const int all = pairs + (frame_last ? 1 : 0);
       bool tiled = false;
-      if (all >= 2 && d->stream != nullptr)
+      if (all >= 2)
         if (lbx_status st = tiled_applies(d, t, &tiled)) return st;
       if (tiled) {
         if (lbx_status st = tiled_pairs(d, t, all, frame_last)) return st;
         t += 2 * all;
         continue;
       }
-      if (pairs >= 2 && d->stream != nullptr) {
+      if (pairs >= 2) {
         if (lbx_status st = replay_pairs(d, t, pairs)) return st;
         t += 2 * pairs;
         continue;
