@@ -1097,13 +1097,7 @@ lbx_status lbx_download_mv(lbx_domain* d, int subs, void* rho, void* ux, void* u
   const size_t plane = (size_t)d->N * d->real_size;
   char* base = (char*)d->mv + (size_t)subs * (1 + d->D) * plane;
   void* dst[4] = {rho, ux, uy, uz};
-  for (int c = 0; c <= d->D;) {
-    // planes that lie behind one another on the host too are one copy
-    int n = 1;
-    while (dst[c] && c + n <= d->D && (char*)dst[c + n] == (char*)dst[c] + n * plane) ++n;
-    if (dst[c]) CK(lbx_internal_copy_out(d->p.device, d->stream, dst[c], base + c * plane, n * plane));
-    c += n;
-  }
+  CK(lbx_internal_copy_planes_out(d->p.device, d->stream, dst, 1 + d->D, base, plane));
   CK(cudaStreamSynchronize(d->stream));
   return LBX_OK;
 }

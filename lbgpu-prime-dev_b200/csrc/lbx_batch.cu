@@ -866,14 +866,7 @@ lbx_status lbx_batch_download_mv(lbx_batch* b, int s, void* rho, void* ux, void*
   const size_t rs = (size_t)b->precision, plane = (size_t)b->N[s] * rs;
   const char* base = (const char*)b->mv + (size_t)b->mvbase[s] * rs;
   void* dst[4] = {rho, ux, uy, uz};
-  for (int c = 0; c <= b->dims;) {
-    // planes that lie behind one another on the host too are one copy
-    int n = 1;
-    while (dst[c] && c + n <= b->dims && (char*)dst[c + n] == (char*)dst[c] + n * plane) ++n;
-    if (dst[c])
-      BCK(lbx_internal_copy_out(b->device, b->stream, dst[c], base + c * plane, n * plane));
-    c += n;
-  }
+  BCK(lbx_internal_copy_planes_out(b->device, b->stream, dst, 1 + b->dims, base, plane));
   BCK(cudaStreamSynchronize(b->stream));
   return LBX_OK;
 }

@@ -221,6 +221,22 @@ cudaError_t lbx_internal_copy_out(int device, cudaStream_t stream, void* dst, co
   return copy(device, stream, dst, src, bytes, true);
 }
 
+cudaError_t lbx_internal_copy_planes_out(int device, cudaStream_t stream, void* const* dst,
+                                         int count, const void* src, size_t plane)
+{
+  for (int c = 0, n = 1; c < count; c += n, n = 1) {
+    if (!dst[c]) continue;
+    if (count * plane >= kStaged)
+      while (c + n < count && dst[c + n] == (char*)dst[c] + n * plane && pageable(dst[c]) &&
+             pageable(dst[c + n]))
+        ++n;
+    const cudaError_t e =
+        copy(device, stream, dst[c], (const char*)src + c * plane, n * plane, true);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 cudaError_t lbx_internal_copy_in(int device, cudaStream_t stream, void* dst, const void* src,
                                  size_t bytes)
 {

@@ -99,11 +99,18 @@ LBX_HIDDEN void lbx_internal_drop_graphs(lbx_domain* d);
 // Copies between device memory and the caller's host buffers, ordered after
 // the stream's earlier work (lbx_copy.cu): staged through page-locked chunks
 // and waited for where that is faster, else queued on the stream.  Each
-// domain and batch registers as a user (add = 1, -1) of its device's chunks.
+// domain and batch registers as a user (copy_user, add = 1, -1) of its
+// device's chunks.
 LBX_HIDDEN cudaError_t lbx_internal_copy_out(int device, cudaStream_t stream, void* dst,
                                              const void* src, size_t bytes);
 LBX_HIDDEN cudaError_t lbx_internal_copy_in(int device, cudaStream_t stream, void* dst,
                                             const void* src, size_t bytes);
+// Planes that lie behind one another at src to dst[c] each (NULL: left out).
+// Planes that lie so on the host too are one copy where their memory is
+// pageable: a copy must not reach from page-locked memory into other.
+LBX_HIDDEN cudaError_t lbx_internal_copy_planes_out(int device, cudaStream_t stream,
+                                                    void* const* dst, int count, const void* src,
+                                                    size_t plane);
 LBX_HIDDEN void lbx_internal_copy_user(int device, int add);
 // PEST sampling: whether a sample is due at time t (the step then writes
 // the macro variables), the gather after that step, and the release.
