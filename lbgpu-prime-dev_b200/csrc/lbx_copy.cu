@@ -1,19 +1,28 @@
 // lbx_copy.cu -- large copies between device memory and the caller's
 // pageable host buffers.
 //
-// A plain copy into a freshly allocated pageable buffer runs at 5 GB/s here:
-// the driver stages it on one thread, which also takes the buffer's page
-// faults (the four macro-variable planes of 150 x 131 x 117 FP64 nodes, 74
-// MB, took 14.6 ms of a 29 ms job; 2.4 ms staged).  Copies of 4 MB or more go
-// through page-locked chunks instead, filled or emptied by several host
-// threads while the next chunks cross the link; a smaller one is done about
-// when the threads have started (0.1 ms).  Smaller copies, buffers the
-// caller has page-locked, and any failure to set this up take the plain copy.
+// A plain copy into a freshly allocated pageable buffer is slow: the driver
+// stages it on one thread, which also takes the buffer's page faults (74 MB,
+// the four macro-variable planes of 150 x 131 x 117 FP64 nodes: 15 to 34 ms,
+// the host's state decides).  Copies of 4 MB or more go through page-locked
+// chunks instead, one for each of several host threads: while one thread
+// empties or fills its chunk the others' cross the link (74 MB to the host:
+// 3.5 ms; as fast with two chunks a thread; chunks of 512 KB 4.5, of 256 KB
+// 5.0).  A smaller copy is done about when the threads have started (0.1 ms).
+// From the host there is less to gain: 18 MB take 0.85 ms, plain 1.0 out of
+// the caches and 2 out of memory.  Smaller copies, buffers the caller has
+// page-locked, and any failure to set this up take the plain copy.
 //
-// The chunks (one set per device, 1 MB x 2 x threads, at most 16 MB) live
-// while any domain or batch of the device does: made by the first large copy,
-// given back when the last is destroyed.  One copy uses them at a time; a
-// copy that finds them taken by another host thread is a plain one.
+// Page-locking costs about 1 ms per MB, so it has to have been earned: the
+// chunks are made when copies that would have gained about as much by them
+// went before (kEarned).  A program that makes a domain, sets its fields and
+// runs does not pay for what it does not use: with the chunks made by the
+// first large copy, that took 20 ms longer.
+//
+// The chunks (one set per device, at most 8 MB) live while any domain or
+// batch of the device does, and are given back when the last is destroyed.
+// One copy uses them at a time; a copy that finds them taken by another host
+// thread is a plain one.
 #include "lbx.h"
 #include "lbx_internal.h"
 
@@ -28,19 +37,25 @@ namespace {
 
 constexpr size_t kChunk = 1 << 20;
 constexpr size_t kStaged = 4 << 20;     // copies from this size on are staged
+// Bytes copied before the chunks are made, those from the host counted an
+// eighth: what the chunks' 8 MB cost in time, plain copies of 16 MB into
+// fresh pages lose against staged ones.
+constexpr size_t kEarned = 16 << 20;
 constexpr int kMaxWorkers = 8;
 
 struct Worker {
-  void* buf[2] = {nullptr, nullptr};
-  cudaEvent_t ev[2] = {nullptr, nullptr};
-  cudaStream_t stream = nullptr;
+  char* buf = nullptr;                  // its part of Stage::chunks
+  cudaEvent_t ev = nullptr;             // its last copy is done
 };
 
 struct Stage {
   std::mutex busy;
   int users = 0;
   bool failed = false;                  // could not be set up: not tried again
+  size_t earned = 0;
+  void* chunks = nullptr;
   std::vector<Worker> workers;
+  cudaStream_t stream = nullptr;        // all chunks': the link carries one after another
   cudaEvent_t ready = nullptr;
 };
 
@@ -49,30 +64,29 @@ std::map<int, Stage> g_stages;          // per device; nodes never move
 
 void tear_down(Stage& s)
 {
-  for (Worker& w : s.workers) {
-    for (int b = 0; b < 2; ++b) {
-      if (w.buf[b]) cudaFreeHost(w.buf[b]);
-      if (w.ev[b]) cudaEventDestroy(w.ev[b]);
-    }
-    if (w.stream) cudaStreamDestroy(w.stream);
-  }
+  for (Worker& w : s.workers)
+    if (w.ev) cudaEventDestroy(w.ev);
   s.workers.clear();
+  if (s.chunks) cudaFreeHost(s.chunks);
+  if (s.stream) cudaStreamDestroy(s.stream);
   if (s.ready) cudaEventDestroy(s.ready);
+  s.chunks = nullptr;
+  s.stream = nullptr;
   s.ready = nullptr;
 }
 
 bool set_up(Stage& s)
 {
-  if (s.failed) return false;
+  if (s.failed || s.earned < kEarned) return false;
   if (!s.workers.empty()) return true;
   const int n = std::min(kMaxWorkers, (int)std::thread::hardware_concurrency() / 2);
-  bool ok = n >= 2 && cudaEventCreateWithFlags(&s.ready, cudaEventDisableTiming) == cudaSuccess;
+  bool ok = n >= 2 && cudaEventCreateWithFlags(&s.ready, cudaEventDisableTiming) == cudaSuccess &&
+            cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) == cudaSuccess &&
+            cudaHostAlloc(&s.chunks, n * kChunk, cudaHostAllocDefault) == cudaSuccess;
   if (ok) s.workers.resize(n);
-  for (Worker& w : s.workers) {
-    ok = ok && cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking) == cudaSuccess;
-    for (int b = 0; b < 2; ++b)
-      ok = ok && cudaHostAlloc(&w.buf[b], kChunk, cudaHostAllocDefault) == cudaSuccess &&
-           cudaEventCreateWithFlags(&w.ev[b], cudaEventDisableTiming) == cudaSuccess;
+  for (size_t w = 0; w < s.workers.size(); ++w) {
+    s.workers[w].buf = (char*)s.chunks + w * kChunk;
+    ok = ok && cudaEventCreateWithFlags(&s.workers[w].ev, cudaEventDisableTiming) == cudaSuccess;
   }
   if (!ok) {
     cudaGetLastError();
@@ -82,39 +96,20 @@ bool set_up(Stage& s)
   return ok;
 }
 
-// Worker w's chunks: w, w + n, w + 2n, ...
-cudaError_t drain(Worker& w, int device, int first, int n, char* dst, const char* src, size_t bytes)
+// One worker's chunks of the copy: first, first + n, first + 2n, ...
+cudaError_t move(Stage& s, int device, int first, int n, char* dst, const char* src, size_t bytes,
+                 bool out)
 {
+  const Worker& w = s.workers[first];
   cudaError_t e = cudaSetDevice(device);
-  const size_t chunks = (bytes + kChunk - 1) / kChunk;
-  auto length = [&](size_t k) { return std::min(kChunk, bytes - k * kChunk); };
-  auto issue = [&](size_t k, int b) {
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(w.buf[b], src + k * kChunk, length(k), cudaMemcpyDeviceToHost, w.stream);
-    if (e == cudaSuccess) e = cudaEventRecord(w.ev[b], w.stream);
-  };
-  int b = 0;
-  if ((size_t)first < chunks) issue(first, 0);
-  for (size_t k = first; k < chunks && e == cudaSuccess; k += n, b ^= 1) {
-    if (k + n < chunks) issue(k + n, b ^ 1);
-    if (e == cudaSuccess) e = cudaEventSynchronize(w.ev[b]);
-    if (e == cudaSuccess) std::memcpy(dst + k * kChunk, w.buf[b], length(k));
-  }
-  return e;
-}
-
-cudaError_t fill(Worker& w, int device, int first, int n, char* dst, const char* src, size_t bytes)
-{
-  cudaError_t e = cudaSetDevice(device);
-  const size_t chunks = (bytes + kChunk - 1) / kChunk;
-  int b = 0;
-  for (size_t k = first, i = 0; k < chunks && e == cudaSuccess; k += n, ++i, b ^= 1) {
-    const size_t len = std::min(kChunk, bytes - k * kChunk);
-    if (i >= 2) e = cudaEventSynchronize(w.ev[b]);     // the chunk's last copy has left
-    if (e != cudaSuccess) break;
-    std::memcpy(w.buf[b], src + k * kChunk, len);
-    e = cudaMemcpyAsync(dst + k * kChunk, w.buf[b], len, cudaMemcpyHostToDevice, w.stream);
-    if (e == cudaSuccess) e = cudaEventRecord(w.ev[b], w.stream);
+  for (size_t at = first * kChunk; at < bytes && e == cudaSuccess; at += n * kChunk) {
+    const size_t len = std::min(kChunk, bytes - at);
+    if (!out) std::memcpy(w.buf, src + at, len);
+    e = out ? cudaMemcpyAsync(w.buf, src + at, len, cudaMemcpyDeviceToHost, s.stream)
+            : cudaMemcpyAsync(dst + at, w.buf, len, cudaMemcpyHostToDevice, s.stream);
+    if (e == cudaSuccess) e = cudaEventRecord(w.ev, s.stream);
+    if (e == cudaSuccess) e = cudaEventSynchronize(w.ev);
+    if (out && e == cudaSuccess) std::memcpy(dst + at, w.buf, len);
   }
   return e;
 }
@@ -138,6 +133,7 @@ bool staged(int device, cudaStream_t stream, void* dst, const void* src, size_t 
   }
   std::unique_lock<std::mutex> lock(s->busy, std::try_to_lock);
   if (!lock.owns_lock()) return false;
+  s->earned += out ? bytes : bytes / 8;
   // streams and events belong to the current device: the domain's, and the
   // caller's again at the end
   struct Current {
@@ -148,13 +144,11 @@ bool staged(int device, cudaStream_t stream, void* dst, const void* src, size_t 
   if (!set_up(*s)) return false;
   const int n = (int)s->workers.size();
   cudaError_t e = cudaEventRecord(s->ready, stream);
-  for (Worker& w : s->workers)
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(w.stream, s->ready, 0);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(s->stream, s->ready, 0);
   std::vector<cudaError_t> res(n, e);
   std::vector<std::thread> threads;
   auto work = [&](int w) {
-    res[w] = out ? drain(s->workers[w], device, w, n, (char*)dst, (const char*)src, bytes)
-                 : fill(s->workers[w], device, w, n, (char*)dst, (const char*)src, bytes);
+    res[w] = move(*s, device, w, n, (char*)dst, (const char*)src, bytes, out);
   };
   if (e == cudaSuccess) {
     threads.reserve(n - 1);
@@ -166,10 +160,8 @@ bool staged(int device, cudaStream_t stream, void* dst, const void* src, size_t 
     for (int w = started + 1; w < n; ++w) work(w);      // threads that could not start
     for (std::thread& t : threads) t.join();
   }
-  for (Worker& w : s->workers) {
-    const cudaError_t f = cudaStreamSynchronize(w.stream);
-    if (e == cudaSuccess) e = f;
-  }
+  const cudaError_t f = cudaStreamSynchronize(s->stream);
+  if (e == cudaSuccess) e = f;
   for (cudaError_t r : res)
     if (e == cudaSuccess) e = r;
   *err = e;
@@ -178,7 +170,7 @@ bool staged(int device, cudaStream_t stream, void* dst, const void* src, size_t 
 
 cudaError_t copy(int device, cudaStream_t stream, void* dst, const void* src, size_t bytes, bool out)
 {
-  // (in a caller's capture the event below would draw the workers' streams in)
+  // (in a caller's capture the event would draw the chunks' stream in)
   if (bytes >= kStaged && pageable(out ? dst : src) && !lbx_internal_capturing(stream)) {
     try {
       cudaError_t e = cudaSuccess;
@@ -212,6 +204,7 @@ void lbx_internal_copy_user(int device, int add)
     // no domain or batch is left on the device, so no copy is under way
     tear_down(s);
     s.failed = false;
+    s.earned = 0;
   } catch (...) {}
 }
 

@@ -1,0 +1,55 @@
+"""The page-locked chunks of large host copies: a program pays for them only
+when it has copied about as much as they cost, and every byte arrives before
+and after they are made."""
+import time
+
+import numpy as np
+import pytest
+
+import lbx
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+def _domain(n):
+    p = lbx.Params(dims=3, LX=n, LY=1, LZ=1, precision=4, layout=lbx.LBX_LAYOUT_DENSE)
+    return lbx.Domain(p, np.zeros(n, np.uint8))
+
+
+def test_one_domain_per_job_does_not_pay_for_chunks():
+    """Jobs that upload 18 MB and look at nothing, from pageable and from
+    page-locked memory (which never needs chunks)."""
+    import torch
+    n = 18 * MB // 4
+    rho = dict(pageable=np.linspace(0.9, 1.1, n, dtype=np.float32),
+               locked=torch.linspace(0.9, 1.1, n).pin_memory().numpy())
+
+    def job(src):
+        at = time.perf_counter()
+        with _domain(n) as d:
+            d.init_equilibrium(0, src)
+        return time.perf_counter() - at
+
+    took = {k: sorted(job(v) for _ in range(7))[3] for k, v in rho.items()}
+    assert took["pageable"] < took["locked"] + 6e-3, took
+
+
+@pytest.mark.parametrize("before", [0, 40 * MB])
+def test_bytes_before_and_after_the_chunks_are_made(before):
+    n0 = 500_000                                        # 38 MB of populations
+    f0 = np.random.default_rng(0).random((1, 19, n0)).astype(np.float32)
+    with _domain(n0) as keep:                           # the chunks live as long
+        keep.upload_f(f0)
+        for _ in range(-(-before // f0.nbytes)):
+            assert np.array_equal(keep.download_f(), f0)
+        # bytes of [19][n] floats around 4 MB and numbers of chunks,
+        # last chunks ragged
+        for n in (4 * MB // 76 + 1, 4 * MB // 76 + 13797 * 3 + 1, 8 * MB // 76, 8 * MB // 76 + 1,
+                  18 * MB // 76 + 17, 41 * MB // 76 + 3):
+            f = np.random.default_rng(n).random((1, 19, n)).astype(np.float32)
+            with _domain(n) as d:
+                d.upload_f(f)
+                assert np.array_equal(d.download_f(), f)
+                assert np.array_equal(d.download_f(), f)
