@@ -424,24 +424,35 @@ struct FluidSums {
       }
     }
   }
-  // fluid nodes in [x0, x1) x [y0, y1), -ext <= x0 <= x1 <= LX + ext (same for y)
-  int rect(int x0, int y0, int x1, int y1) const
+};
+
+// One column of tiles: fluid nodes in the rows below y (from -ext on) of the
+// column widened by j on both sides, for the three j that work() asks for.
+struct Band {
+  int K, ext;
+  std::vector<int> s[3];
+
+  Band(const FluidSums& fs, int x, int w, int k) : K(k), ext(fs.ext)
   {
-    x0 += ext; x1 += ext; y0 += ext; y1 += ext;
-    return s[(size_t)y1 * W + x1] - s[(size_t)y0 * W + x1] - s[(size_t)y1 * W + x0] +
-           s[(size_t)y0 * W + x0];
+    for (int q = 0; q < 3; ++q) {
+      const int j = ring(q), rows = fs.LY + 2 * ext + 1;
+      s[q].resize(rows);
+      const int* p = fs.s.data() + x - j + ext;
+      for (int y = 0; y < rows; ++y, p += fs.W) s[q][y] = p[w + 2 * j] - p[0];
+    }
   }
-  // fluid nodes within j of the tile (x0, y0, w, h)
-  long long around(int x0, int y0, int w, int h, int j) const
+  int ring(int q) const { return q == 0 ? 0 : q == 1 ? (K - 1) / 2 : K - 1; }
+  // fluid nodes within ring(q) of the tile of rows [y, y + h)
+  long long around(int q, int y, int h) const
   {
-    return rect(x0 - j, y0 - j, x0 + w + j, y0 + h + j);
+    return s[q][y + h + ring(q) + ext] - s[q][y - ring(q) + ext];
   }
-  // node updates of one round of a tile, about: the sum of around(j) over
-  // j = 0 .. K - 1 by Simpson's rule (exact where the fluid is uniform)
-  long long work(int x0, int y0, int w, int h, int K) const
+  // node updates of one round of the tile, about: the sum of the fluid nodes
+  // within j over j = 0 .. K - 1 by Simpson's rule (exact where the fluid is
+  // uniform)
+  long long work(int y, int h) const
   {
-    return K * (around(x0, y0, w, h, 0) + 4 * around(x0, y0, w, h, (K - 1) / 2) +
-                around(x0, y0, w, h, K - 1)) / 6;
+    return K * (around(0, y, h) + 4 * around(1, y, h) + around(2, y, h)) / 6;
   }
 };
 
@@ -520,22 +531,28 @@ int best_shapes(int LX, int LY, double fluid, int blocks, Shape (&best)[kShapes]
   return n;
 }
 
-// Tiles of about equal work for a shape; false when a halo reads too many.
+// Tiles of about equal work for a shape, column by column from the first row
+// up; false when a halo reads too many.
 bool make_tiles(const FluidSums& fs, int LX, int LY, const Shape& sh, int cap,
                 std::vector<Tile>& tiles, std::vector<int>& nbrs)
 {
   const int K = sh.K;
   auto edge = [&](int c) { return (int)((long long)LX * c / sh.cols); };
+  std::vector<Band> bands;
+  bands.reserve(sh.cols);
+  for (int c = 0; c < sh.cols; ++c) bands.emplace_back(fs, edge(c), edge(c + 1) - edge(c), K);
+  std::vector<int> first(sh.cols + 1);                // a column's first tile
   auto cut = [&](long long W, std::vector<Tile>* to) -> bool {
     int n = 0;
     for (int c = 0; c < sh.cols && n <= sh.tiles; ++c) {
       const int x = edge(c), w = edge(c + 1) - x;
       const int hmax = cap / tiled_pitch(w, K) - 2 * K;
+      first[c] = n;
       for (int y = 0; y < LY && n <= sh.tiles; ++n) {
         int h = 1, most = std::min(hmax, LY - y);     // the work grows with h
         while (h < most) {
           const int mid = (h + most + 1) / 2;
-          if (fs.work(x, y, w, mid, K) <= W) h = mid; else most = mid - 1;
+          if (bands[c].work(y, mid) <= W) h = mid; else most = mid - 1;
         }
         if (to) {
           Tile t;
@@ -546,12 +563,12 @@ bool make_tiles(const FluidSums& fs, int LX, int LY, const Shape& sh, int cap,
         y += h;
       }
     }
+    first[sh.cols] = n;
     return n <= sh.tiles;
   };
   // about the least work bound that needs no more tiles (to 2 %)
   long long hi = 0;
-  for (int c = 0; c < sh.cols; ++c)
-    hi += fs.work(edge(c), 0, edge(c + 1) - edge(c), (LY + sh.rows - 1) / sh.rows, K);
+  for (int c = 0; c < sh.cols; ++c) hi += bands[c].work(0, (LY + sh.rows - 1) / sh.rows);
   hi = hi / sh.cols + 1;
   long long lo = 0;
   while (!cut(hi, nullptr)) {
@@ -565,33 +582,42 @@ bool make_tiles(const FluidSums& fs, int LX, int LY, const Shape& sh, int cap,
   }
   tiles.clear();
   cut(hi, &tiles);
-  // the tiles each halo reads: its columns, each looked at once per row
-  std::vector<int> column(LX), owner((size_t)sh.cols * LY);
+  // the tiles each halo reads: the columns around the tile's, in each the
+  // tiles around its rows, from the one that holds the halo's first row up;
+  // a halo that goes round the lattice meets a tile again
+  std::vector<int> owner((size_t)sh.cols * LY);
   for (int c = 0; c < sh.cols; ++c)
-    for (int x = edge(c); x < edge(c + 1); ++x) column[x] = c;
-  for (size_t t = 0; t < tiles.size(); ++t)
-    for (int y = tiles[t].y; y < tiles[t].y + tiles[t].h; ++y)
-      owner[(size_t)column[tiles[t].x] * LY + y] = (int)t;
+    for (int t = first[c]; t < first[c + 1]; ++t)
+      std::fill_n(owner.begin() + (size_t)c * LY + tiles[t].y, tiles[t].h, t);
   nbrs.assign(tiles.size() * kMaxNb, -1);
-  std::vector<int> cols;
-  for (size_t t = 0; t < tiles.size(); ++t) {
-    const Tile& g = tiles[t];
-    cols.clear();
-    for (int x = g.x - K; x < g.x + g.w + K; ++x) {
-      const int c = column[(x % LX + LX) % LX];
-      if (cols.empty() || cols.back() != c) cols.push_back(c);
+  std::vector<int> met(tiles.size(), -1);
+  for (int c = 0, t = 0; c < sh.cols; ++c) {
+    int c0 = c, left = K;                             // the column of the halo's first node
+    for (int n = 1; left > 0 && n < sh.cols; ++n) {
+      c0 = c0 == 0 ? sh.cols - 1 : c0 - 1;
+      left -= edge(c0 + 1) - edge(c0);
     }
-    int k = 0;
-    int* const row = &nbrs[t * kMaxNb];
-    for (int c : cols)
-      for (int y = g.y - K, last = -1; y < g.y + g.h + K; ++y) {
-        const int o = owner[(size_t)c * LY + (y % LY + LY) % LY];
-        if (o == last) continue;
-        last = o;
-        if (std::find(row, row + k, o) != row + k) continue;
-        if (k == kMaxNb) return false;
-        row[k++] = o;
+    int across = 0;                                   // columns from there on
+    for (int w = left > 0 ? LX : K - left + edge(c + 1) - edge(c) + K, q = c0;
+         w > 0 && across < sh.cols; ++across, q = q + 1 == sh.cols ? 0 : q + 1)
+      w -= edge(q + 1) - edge(q);
+    for (; t < first[c + 1]; ++t) {
+      const Tile& g = tiles[t];
+      int y0 = (g.y - K) % LY;
+      if (y0 < 0) y0 += LY;
+      int k = 0;
+      int* const row = &nbrs[(size_t)t * kMaxNb];
+      for (int i = 0, q = c0; i < across; ++i, q = q + 1 == sh.cols ? 0 : q + 1) {
+        int o = owner[(size_t)q * LY + y0];
+        for (int rows = y0 - tiles[o].y + g.h + 2 * K; rows > 0 && met[o] != t;) {
+          met[o] = t;
+          if (k == kMaxNb) return false;
+          row[k++] = o;
+          rows -= tiles[o].h;
+          if (++o == first[q + 1]) o = first[q];
+        }
       }
+    }
   }
   return true;
 }
