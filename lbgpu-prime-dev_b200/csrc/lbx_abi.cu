@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <new>
 #include <type_traits>
 #include <vector>
 
@@ -846,8 +847,8 @@ lbx_status replay_pairs(lbx_domain* d, int t, int pairs)
 }
 
 // Whether the tiled path takes a stretch of AA pairs starting at odd time t
-// with unchanging arguments; LBX_RUN_AUTO asks its plan whether it is the
-// faster one (lbx_tiled.cu), LBX_RUN_TILED only whether it applies.
+// with unchanging arguments: LBX_RUN_AUTO where it is modelled the faster one
+// (lbx_tiled.cu), LBX_RUN_TILED wherever it applies.
 lbx_status tiled_applies(lbx_domain* d, int t, bool* yes)
 {
   const lbx_params& p = d->p;
@@ -855,10 +856,7 @@ lbx_status tiled_applies(lbx_domain* d, int t, bool* yes)
   if (d->run_mode == LBX_RUN_STEPS || d->tiled_state < 0) return LBX_OK;
   if (p.dims != 2 || d->ns || d->btc_vals || d->fout) return LBX_OK;
   if (d->faces_active && (!d->faces_fused || solute_faces_idle(d, t))) return LBX_OK;
-  bool better = false;
-  if (lbx_status st = lbx_internal_tiled_plan(d, &better)) return st;
-  *yes = d->tiled_state > 0 && (better || d->run_mode == LBX_RUN_TILED);
-  return LBX_OK;
+  return lbx_internal_tiled_plan(d, yes);
 }
 
 lbx_status tiled_pairs(lbx_domain* d, int t, int pairs, bool write_mv)
@@ -952,7 +950,9 @@ lbx_status lbx_create(const lbx_params* p, const uint8_t* solids, lbx_domain** o
                   : p->layout;
 
   // the tiled run's plan reads the mask (lbx_tiled.cu; no larger lattice fits)
-  if (p->dims == 2 && d->N <= (1 << 20)) d->host_solids.assign(solids, solids + d->N);
+  try {
+    if (p->dims == 2 && d->N <= (1 << 20)) d->host_solids.assign(solids, solids + d->N);
+  } catch (const std::bad_alloc&) {}    // then it is not planned
 
   auto bail = [&](lbx_status s) { release(d); delete d; return s; };
   cudaError_t e;
@@ -970,10 +970,18 @@ lbx_status lbx_create(const lbx_params* p, const uint8_t* solids, lbx_domain** o
   const size_t fbytes = (size_t)p->nsubs * d->Q * d->N * d->real_size;
   const size_t mvbytes = (size_t)p->nsubs * (1 + d->D) * d->N * d->real_size;
   if (d->layout == LBX_LAYOUT_COMPACT) d->P = (d->fluid + 31) / 32 * 32;
+  // a population array, with room for the tiled run behind it if it can be had
   const size_t tiled_room = p->walsh ? 0 : lbx_internal_tiled_room(d);
-  const size_t tiled_dense = d->layout == LBX_LAYOUT_COMPACT ? 0 : tiled_room;
-  CKD(cudaMalloc(&d->f, (fbytes + 255) / 256 * 256 + tiled_dense));
-  if (tiled_dense) d->tiled_room = (char*)d->f + (fbytes + 255) / 256 * 256;
+  auto alloc_f = [&](void** f, size_t bytes, size_t room) {
+    const size_t at = (bytes + 255) / 256 * 256;
+    if (room && cudaMalloc(f, at + room) == cudaSuccess) {
+      d->tiled_room = (char*)*f + at;
+      return cudaSuccess;
+    }
+    if (room) cudaGetLastError();
+    return cudaMalloc(f, std::max<size_t>(1, bytes));
+  };
+  CKD(alloc_f(&d->f, fbytes, d->layout == LBX_LAYOUT_COMPACT ? 0 : tiled_room));
   CKD(cudaMalloc(&d->mv, mvbytes));
   CKD(cudaMalloc(&d->solids, d->N));
   CKD(cudaMalloc(&d->cls, d->N));
@@ -988,8 +996,7 @@ lbx_status lbx_create(const lbx_params* p, const uint8_t* solids, lbx_domain** o
       else { fidx[n] = m; fnode[m++] = (int)n; }
     }
     const size_t fcbytes = (size_t)p->nsubs * d->Q * d->P * d->real_size;
-    CKD(cudaMalloc(&d->fc, std::max<size_t>(1, (fcbytes + 255) / 256 * 256 + tiled_room)));
-    if (tiled_room) d->tiled_room = (char*)d->fc + (fcbytes + 255) / 256 * 256;
+    CKD(alloc_f(&d->fc, fcbytes, tiled_room));
     CKD(cudaMalloc(&d->fidx, d->N * sizeof(int)));
     CKD(cudaMalloc(&d->fnode, fnode.size() * sizeof(int)));
     CKD(cudaMemcpy(d->fidx, fidx.data(), d->N * sizeof(int), cudaMemcpyHostToDevice));

@@ -72,7 +72,7 @@ struct lbx_domain {
   std::vector<uint8_t> host_solids;      // 2D lattices the tiles may fit: the mask, for the plan
   int tiled_state = 0;                   // 0: not planned, 1: planned, -1: no tiles fit
   int tiled_k = 0;                       // steps per round, at most
-  double tiled_us = 0.0;                 // modelled time per step
+  double tiled_us = 1e30;                // modelled time per step of its best tiles
   void* tiled_room = nullptr;            // memory for the two below, behind the population array
   void* tiled_own = nullptr;             // or allocated by the plan
   void* tiled_scratch = nullptr;         // a second population array for its rounds
@@ -117,17 +117,15 @@ LBX_HIDDEN void lbx_internal_copy_user(int device, int add);
 LBX_HIDDEN bool lbx_internal_pest_due(const lbx_domain* d, int t);
 LBX_HIDDEN lbx_status lbx_internal_pest_after(lbx_domain* d, int t);
 LBX_HIDDEN void lbx_internal_pest_free(lbx_domain* d);
-// Temporal blocking: plans the tiles on first use (tiled_state tells whether
-// they fit) and tells whether the tiled run is modelled faster than a launch
-// per step; then `pairs` AA pairs (two or more) with the launch arguments A
-// from the state after an even step, the last step writing the macro
-// variables if asked.
-// Bytes the tiled run of this lattice would like behind the population
-// array (0: it would not be taken).
-LBX_HIDDEN size_t lbx_internal_tiled_room(const lbx_domain* d);
+// Temporal blocking.  At creation: bytes the tiled run of this lattice would
+// like behind the population array (0: it would not be taken).  Then whether
+// the domain's run mode takes it, the tiles planned on first use; then
+// `pairs` AA pairs (two or more) with the launch arguments A from the state
+// after an even step, the last step writing the macro variables if asked.
+LBX_HIDDEN size_t lbx_internal_tiled_room(lbx_domain* d);
 // Whether the caller is capturing `stream` into a graph of its own.
 LBX_HIDDEN bool lbx_internal_capturing(cudaStream_t stream);
-LBX_HIDDEN lbx_status lbx_internal_tiled_plan(lbx_domain* d, bool* better);
+LBX_HIDDEN lbx_status lbx_internal_tiled_plan(lbx_domain* d, bool* yes);
 template <typename T>
 LBX_HIDDEN lbx_status lbx_internal_tiled_run(lbx_domain* d, const lbx::StepArgs<T>& A, int pairs,
                                              bool write_mv);

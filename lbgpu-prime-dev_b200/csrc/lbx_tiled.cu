@@ -52,6 +52,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <new>
 #include <vector>
 
 using namespace lbx;
@@ -643,13 +644,23 @@ size_t tables_bytes(int tiles, size_t nodes)
          nodes * (sizeof(int) + 3 * sizeof(unsigned short));
 }
 
+bool better(const lbx_domain* d)
+{
+  return d->tiled_us < steps_us((double)d->fluid, d->real_size, d->p.nsubs);
+}
+
+// The room a tiled run of the lattice wants, 0 where it is modelled slower
+// than a launch per step (tiled_us, looked for once); tiled_state -1 where
+// no shape fits.
 template <typename T, int NS>
-size_t room(const lbx_domain* d, int blocks)
+size_t room(lbx_domain* d, int blocks)
 {
   Shape shapes[kShapes];
   const double fluid = (double)d->fluid / (double)d->N;
   const int n = best_shapes<T, NS>(d->p.LX, d->p.LY, fluid, blocks, shapes);
-  if (n == 0 || shapes[0].us >= steps_us((double)d->fluid, d->real_size, NS)) return 0;
+  if (n == 0) { d->tiled_state = -1; return 0; }
+  d->tiled_us = shapes[0].us;
+  if (!better(d)) return 0;
   size_t most = 0;
   for (int i = 0; i < n; ++i)
     most = std::max(most, tables_bytes(shapes[i].tiles, region_nodes(shapes[i], d->p.LX, d->p.LY)));
@@ -657,8 +668,7 @@ size_t room(const lbx_domain* d, int blocks)
 }
 
 // Plans the lattice's tiles and makes their tables, once per domain:
-// tiled_state 1, or -1 where no shape fits; it stays 0 where one fits but
-// the launch-per-step path is modelled faster and the run mode does not ask.
+// tiled_state 1, or -1 where no shape fits or there is no memory for it.
 template <typename T, int NS>
 lbx_status make_plan(lbx_domain* d)
 {
@@ -671,12 +681,6 @@ lbx_status make_plan(lbx_domain* d)
   const double fluid = (double)d->fluid / (double)d->N;
   Shape shapes[kShapes];
   const int ns = best_shapes<T, NS>(p.LX, p.LY, fluid, sms, shapes);
-  // not worth a plan unless some run mode would take it
-  if (ns == 0 || (d->run_mode != LBX_RUN_TILED &&
-                  shapes[0].us >= steps_us((double)d->fluid, d->real_size, p.nsubs))) {
-    d->tiled_state = ns == 0 ? -1 : 0;
-    return LBX_OK;
-  }
   const FluidSums fs(d->host_solids, p.LX, p.LY, kMaxK);
   constexpr int cap = tiled_cap<T, NS>();
   std::vector<Tile> tiles;
@@ -728,6 +732,10 @@ lbx_status make_plan(lbx_domain* d)
   if (e != cudaSuccess) {
     lbx_internal_tiled_free(d);
     d->tiled_state = -1;
+    if (e == cudaErrorMemoryAllocation && d->run_mode != LBX_RUN_TILED) {
+      cudaGetLastError();             // a launch per step needs none
+      return LBX_OK;
+    }
     return lbx_internal_fail(e == cudaErrorMemoryAllocation ? LBX_ERR_NOMEM : LBX_ERR_CUDA,
                              cudaGetErrorString(e));
   }
@@ -791,7 +799,7 @@ lbx_status run_ns(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
 
 }  // namespace
 
-size_t lbx_internal_tiled_room(const lbx_domain* d)
+size_t lbx_internal_tiled_room(lbx_domain* d)
 {
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->p.device) != cudaSuccess) {
@@ -803,18 +811,20 @@ size_t lbx_internal_tiled_room(const lbx_domain* d)
   return d->p.nsubs == 2 ? room<float, 2>(d, sms) : room<float, 1>(d, sms);
 }
 
-lbx_status lbx_internal_tiled_plan(lbx_domain* d, bool* better)
+lbx_status lbx_internal_tiled_plan(lbx_domain* d, bool* yes)
 {
   const lbx_params& p = d->p;
-  *better = false;
-  if (d->tiled_state == 0 && !d->host_solids.empty()) {
+  *yes = false;
+  if (d->host_solids.empty() || (d->run_mode != LBX_RUN_TILED && !better(d))) return LBX_OK;
+  if (d->tiled_state == 0) try {
     lbx_status st = d->real_size == 8
                         ? (p.nsubs == 2 ? make_plan<double, 2>(d) : make_plan<double, 1>(d))
                         : (p.nsubs == 2 ? make_plan<float, 2>(d) : make_plan<float, 1>(d));
     if (st != LBX_OK) return st;
+  } catch (const std::bad_alloc&) {
+    d->tiled_state = -1;              // no host memory for it either
   }
-  *better = d->tiled_state > 0 &&
-            d->tiled_us < steps_us((double)d->fluid, d->real_size, p.nsubs);
+  *yes = d->tiled_state > 0;
   return LBX_OK;
 }
 
