@@ -800,7 +800,9 @@ lbx_status capture_pairs(lbx_domain* d, int t, int npairs, cudaGraphExec_t* out,
 // of the GPU, and capturing the graphs would hold it up (1-2 ms for a step
 // with z faces and a record, the GPU time of 30 such steps at 128 x 112 x
 // 96).  Populations of 50 MB (100 moved) step in some 20 us, more than the
-// launches of a step with faces take.
+// launches of a step with faces take.  Stretches that add up to more pairs
+// with the same arguments throughout have earned the capture: it is the
+// program's loop.
 constexpr int kGraphPairs = 8;
 constexpr int kDirectPairs = 64;
 constexpr double kDirectBytes = 50e6;
@@ -816,7 +818,13 @@ lbx_status replay_pairs(lbx_domain* d, int t, int pairs)
       std::memcmp(d->graph_key, key, klen) != 0) {
     const double bytes = (double)d->p.nsubs * d->Q * (double)d->real_size *
                          (double)(d->layout == LBX_LAYOUT_COMPACT ? d->fluid : d->N);
-    if (pairs < kDirectPairs && bytes > kDirectBytes) {
+    const bool again = d->direct_stream == d->stream && d->direct_key_len == klen &&
+                       std::memcmp(d->direct_key, key, klen) == 0;
+    d->direct_pairs = (again ? d->direct_pairs : 0) + pairs;
+    if (d->direct_pairs < kDirectPairs && bytes > kDirectBytes) {
+      std::memcpy(d->direct_key, key, klen);
+      d->direct_key_len = klen;
+      d->direct_stream = d->stream;
       for (int q = 0; q < 2 * pairs; ++q)
         if (lbx_status st = do_step(d, t + q, 0)) return st;
       return LBX_OK;

@@ -67,6 +67,11 @@ struct lbx_domain {
   unsigned char graph_key[2 * 640];      // keys of the odd and the even step
   size_t graph_key_len = 0;
   long long graph_launches = 0;          // kernels one replay of the graph runs
+  // the last stretch launched directly, and the pairs so far with its arguments
+  cudaStream_t direct_stream = nullptr;
+  unsigned char direct_key[2 * 640];
+  size_t direct_key_len = 0;
+  long long direct_pairs = 0;
   // temporal blocking of small 2D lattices (lbx_tiled.cu)
   int run_mode = LBX_RUN_AUTO;
   std::vector<uint8_t> host_solids;      // 2D lattices the tiles may fit: the mask, for the plan
