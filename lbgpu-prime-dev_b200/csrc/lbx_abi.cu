@@ -861,7 +861,7 @@ lbx_status tiled_applies(lbx_domain* d, int t, bool* yes)
 {
   const lbx_params& p = d->p;
   *yes = false;
-  if (d->run_mode == LBX_RUN_STEPS || d->tiled_state < 0) return LBX_OK;
+  if (d->run_mode == LBX_RUN_STEPS || d->tiled[0].state < 0) return LBX_OK;
   if (p.dims != 2 || d->ns || d->btc_vals || d->fout) return LBX_OK;
   if (d->faces_active && (!d->faces_fused || solute_faces_idle(d, t))) return LBX_OK;
   return lbx_internal_tiled_plan(d, yes);

@@ -8,6 +8,24 @@
 
 #include <vector>
 
+// A division of a small 2D lattice into tiles for one part of the GPU (level
+// l: at most one of its 2^l equal parts), and its tables on the device.
+struct TiledPlan {
+  static constexpr int kLevels = 5;
+  int state = 0;                         // 0: not planned, 1: planned, -1: no tiles fit
+  double us = 0.0;                       // modelled time per step (0: not looked for)
+  int K = 0;                             // steps per round, at most
+  int ntiles = 0;
+  size_t nodes = 0;                      // region nodes of all tiles
+  int base = 0;                          // counter value the next launch starts from
+  void* own = nullptr;                   // its memory, where it has its own
+  void* tiles = nullptr;
+  int* nbrs = nullptr;                   // per tile: the tiles its halo reads
+  int* flags = nullptr;                  // per-tile round counters
+  int* gidx = nullptr;                   // per tile: population slots of its region's nodes
+  unsigned short* list = nullptr;        // per tile: its node list; then the flags words, the halo list
+};
+
 struct lbx_domain {
   lbx_params p;
   int Q = 0, D = 0;
@@ -75,20 +93,19 @@ struct lbx_domain {
   // temporal blocking of small 2D lattices (lbx_tiled.cu)
   int run_mode = LBX_RUN_AUTO;
   std::vector<uint8_t> host_solids;      // 2D lattices the tiles may fit: the mask, for the plan
-  int tiled_state = 0;                   // 0: not planned, 1: planned, -1: no tiles fit
-  int tiled_k = 0;                       // steps per round, at most
-  double tiled_us = 1e30;                // modelled time per step of its best tiles
-  void* tiled_room = nullptr;            // memory for the two below, behind the population array
-  void* tiled_own = nullptr;             // or allocated by the plan
+  TiledPlan tiled[TiledPlan::kLevels];
+  void* tiled_room = nullptr;            // memory for what follows, behind the population array
+  void* tiled_own = nullptr;             // or allocated when first needed
   void* tiled_scratch = nullptr;         // a second population array for its rounds
-  void* tiled_plan = nullptr;            // the tiles, then the tables
-  int* tiled_nbrs = nullptr;             // per tile: the tiles its halo reads
-  int* tiled_gidx = nullptr;             // per tile: population slots of its region's nodes
-  int* tiled_flags = nullptr;            // per-tile round counters, then a status word
-  unsigned short* tiled_list = nullptr;  // per tile: its node list; then the flags words, the halo list
-  int tiled_ntiles = 0;
-  size_t tiled_nodes = 0;                // region nodes of all tiles
-  int tiled_base = 0;                    // counter value the next launch starts from
+  int* tiled_status = nullptr;           // set by a launch whose wait ran out
+  void* tiled_tables = nullptr;          // room for the first plan's tables
+  // its last launch, for other domains' (guarded by the mutex in lbx_tiled.cu,
+  // but for the event itself)
+  cudaEvent_t tiled_done = nullptr;
+  cudaStream_t tiled_stream = nullptr;
+  unsigned long long tiled_turn = 0;
+  bool tiled_listed = false, tiled_busy = false;
+  int tiled_company = 0;                 // others' runs seen beside it
   bool tiled_attr = false;               // the kernel's shared-memory limit is raised
 };
 

@@ -52,6 +52,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -253,9 +254,13 @@ aa_tiled(StepArgs<T> A, TiledArgs<T> R)
           const int nb = R.nbrs[blockIdx.x * kMaxNb + q];
           if (nb < 0) break;
           long long polls = 0;
-          // every poll is an L2 round trip: no sleep between polls
+          // every poll is an L2 round trip: no sleep between polls, and the
+          // status word, a second one, only now and then
           while (observe(R.flags + nb) < R.base + r) {
-            if (++polls >= kWaitLimit || *(volatile int*)R.status != 0) { late = 1; break; }
+            if (++polls >= kWaitLimit || (polls % 64 == 0 && *(volatile int*)R.status != 0)) {
+              late = 1;
+              break;
+            }
           }
         }
         late = __any_sync(0xffffffffu, late);
@@ -630,36 +635,56 @@ size_t region_nodes(const Shape& sh, int LX, int LY)
          ((size_t)sh.cols * LY + (size_t)sh.tiles * 2 * sh.K);
 }
 
-// Bytes of a plan's scratch array, and of its tables: tiles, neighbours,
-// counters and status, then per region node a slot and three list entries.
+// Bytes of the scratch array with the status word behind it, and of a plan's
+// tables: tiles, neighbours, counters, then per region node a slot and three
+// list entries.
 size_t scratch_bytes(const lbx_domain* d)
 {
   const long long P = d->layout == LBX_LAYOUT_COMPACT ? d->P : d->N;
-  return ((size_t)d->p.nsubs * 9 * P * d->real_size + 255) / 256 * 256;
+  return ((size_t)d->p.nsubs * 9 * P * d->real_size + 255) / 256 * 256 + 256;
 }
 
 size_t tables_bytes(int tiles, size_t nodes)
 {
-  return (size_t)tiles * (sizeof(Tile) + (kMaxNb + 1) * sizeof(int)) + sizeof(int) +
+  return (size_t)tiles * (sizeof(Tile) + (kMaxNb + 1) * sizeof(int)) +
          nodes * (sizeof(int) + 3 * sizeof(unsigned short));
 }
 
-bool better(const lbx_domain* d)
+int multiprocessors(const lbx_domain* d)
 {
-  return d->tiled_us < steps_us((double)d->fluid, d->real_size, d->p.nsubs);
+  int sms = 0, coop = 0;
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, d->p.device);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->p.device);
+  if (coop && sms > 0) return sms;
+  cudaGetLastError();
+  return 0;
 }
 
-// The room a tiled run of the lattice wants, 0 where it is modelled slower
-// than a launch per step (tiled_us, looked for once); tiled_state -1 where
-// no shape fits.
+// The best shapes for level l, and their modelled time in the plan; state -1
+// where none fits.
 template <typename T, int NS>
-size_t room(lbx_domain* d, int blocks)
+int shapes_of(lbx_domain* d, int l, Shape (&shapes)[kShapes])
+{
+  const double fluid = (double)d->fluid / (double)d->N;
+  const int n = best_shapes<T, NS>(d->p.LX, d->p.LY, fluid, multiprocessors(d) >> l, shapes);
+  if (n == 0) d->tiled[l].state = -1;
+  d->tiled[l].us = n == 0 ? 1e30 : shapes[0].us;
+  return n;
+}
+
+// Whether the tiled run with the GPU to itself is modelled faster than a
+// launch per step.
+bool better(const lbx_domain* d)
+{
+  const double us = d->tiled[0].us;
+  return us > 0.0 && us < steps_us((double)d->fluid, d->real_size, d->p.nsubs);
+}
+
+template <typename T, int NS>
+size_t room(lbx_domain* d)
 {
   Shape shapes[kShapes];
-  const double fluid = (double)d->fluid / (double)d->N;
-  const int n = best_shapes<T, NS>(d->p.LX, d->p.LY, fluid, blocks, shapes);
-  if (n == 0) { d->tiled_state = -1; return 0; }
-  d->tiled_us = shapes[0].us;
+  const int n = shapes_of<T, NS>(d, 0, shapes);
   if (!better(d)) return 0;
   size_t most = 0;
   for (int i = 0; i < n; ++i)
@@ -667,20 +692,17 @@ size_t room(lbx_domain* d, int blocks)
   return scratch_bytes(d) + most;
 }
 
-// Plans the lattice's tiles and makes their tables, once per domain:
-// tiled_state 1, or -1 where no shape fits or there is no memory for it.
+// Plans the lattice's tiles for level l and makes their tables: state 1, or
+// -1 where no shape fits or there is no memory for it.
 template <typename T, int NS>
-lbx_status make_plan(lbx_domain* d)
+lbx_status make_plan(lbx_domain* d, int l)
 {
   const lbx_params& p = d->p;
-  d->tiled_state = -1;
-  int sms = 0, coop = 0;
-  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, p.device);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p.device);
-  if (!coop || sms < 1 || d->fluid == 0) { cudaGetLastError(); return LBX_OK; }
-  const double fluid = (double)d->fluid / (double)d->N;
+  TiledPlan& plan = d->tiled[l];
   Shape shapes[kShapes];
-  const int ns = best_shapes<T, NS>(p.LX, p.LY, fluid, sms, shapes);
+  const int ns = d->fluid == 0 ? 0 : shapes_of<T, NS>(d, l, shapes);
+  plan.state = -1;
+  if (ns == 0) return LBX_OK;
   const FluidSums fs(d->host_solids, p.LX, p.LY, kMaxK);
   constexpr int cap = tiled_cap<T, NS>();
   std::vector<Tile> tiles;
@@ -689,57 +711,198 @@ lbx_status make_plan(lbx_domain* d)
   while (i < ns && !make_tiles(fs, p.LX, p.LY, shapes[i], cap, tiles, nbrs)) ++i;
   if (i == ns) return LBX_OK;
   const int nt = (int)tiles.size();
-  d->tiled_k = shapes[i].K;
-  d->tiled_us = shapes[i].us;
-  d->tiled_ntiles = nt;
-  d->tiled_base = 0;
+  plan.K = shapes[i].K;
+  plan.us = shapes[i].us;
+  plan.ntiles = nt;
+  plan.base = 0;
   size_t nodes = 0;
   for (Tile& t : tiles) {
     t.at = (int)nodes;
-    nodes += (size_t)tiled_pitch(t.w, d->tiled_k) * (t.h + 2 * d->tiled_k);
+    nodes += (size_t)tiled_pitch(t.w, plan.K) * (t.h + 2 * plan.K);
   }
+  plan.nodes = nodes;
   const size_t b_tiles = (size_t)nt * sizeof(Tile), b_nbrs = nbrs.size() * sizeof(int);
-  const size_t b_flags = (size_t)(nt + 1) * sizeof(int), b_gidx = nodes * sizeof(int);
-  std::vector<char> head(b_tiles + b_nbrs + b_flags, 0);   // counters and status start at 0
+  const size_t b_flags = (size_t)nt * sizeof(int), b_gidx = nodes * sizeof(int);
+  std::vector<char> head(b_tiles + b_nbrs + b_flags, 0);   // counters start at 0
   std::memcpy(head.data(), tiles.data(), b_tiles);
   std::memcpy(head.data() + b_tiles, nbrs.data(), b_nbrs);
-  // the scratch array, then the tables: behind the population array where
-  // lbx_create left room (a call here costs 0.4 ms), else on their own
+  // the scratch array, once, and the tables of level 0: behind the population
+  // array where lbx_create left room (a call here costs 0.4 ms), else on
+  // their own; other levels' tables on their own
   const size_t scratch = scratch_bytes(d);
   cudaError_t e = cudaSuccess;
-  if (!d->tiled_room) {
-    e = cudaMalloc(&d->tiled_own, scratch + tables_bytes(nt, nodes));
-    d->tiled_room = d->tiled_own;
+  if (!d->tiled_scratch) {
+    char* at = (char*)d->tiled_room;
+    if (at) {
+      d->tiled_tables = at + scratch;
+    } else {
+      e = cudaMalloc(&d->tiled_own, scratch);
+      at = (char*)d->tiled_own;
+    }
+    if (e == cudaSuccess) {
+      d->tiled_scratch = at;
+      d->tiled_status = (int*)(at + scratch - 256);
+      e = cudaMemsetAsync(d->tiled_status, 0, sizeof(int), d->stream);
+    }
   }
-  d->tiled_scratch = d->tiled_room;
-  char* at = (char*)d->tiled_room + scratch;
-  d->tiled_plan = at;
-  d->tiled_nbrs = (int*)(at + b_tiles);
-  d->tiled_flags = (int*)(at + b_tiles + b_nbrs);
-  d->tiled_gidx = (int*)(at + b_tiles + b_nbrs + b_flags);
-  d->tiled_list = (unsigned short*)(at + b_tiles + b_nbrs + b_flags + b_gidx);
-  d->tiled_nodes = nodes;
-  if (e == cudaSuccess)
+  char* at = nullptr;
+  if (l == 0 && d->tiled_tables) {
+    at = (char*)d->tiled_tables;
+  } else if (e == cudaSuccess) {
+    e = cudaMalloc(&plan.own, tables_bytes(nt, nodes));
+    at = (char*)plan.own;
+  }
+  if (e == cudaSuccess) {
+    plan.tiles = at;
+    plan.nbrs = (int*)(at + b_tiles);
+    plan.flags = (int*)(at + b_tiles + b_nbrs);
+    plan.gidx = (int*)(at + b_tiles + b_nbrs + b_flags);
+    plan.list = (unsigned short*)(at + b_tiles + b_nbrs + b_flags + b_gidx);
     e = cudaMemcpyAsync(at, head.data(), head.size(), cudaMemcpyHostToDevice, d->stream);
+  }
   if (e == cudaSuccess) {
     tile_tables<<<nt, kTiledThreads, (size_t)cap * sizeof(unsigned short), d->stream>>>(
-        d->cls, d->layout == LBX_LAYOUT_COMPACT ? d->fidx : nullptr, p.LX, p.LY, d->tiled_k,
-        (Tile*)d->tiled_plan, d->tiled_gidx, d->tiled_list, d->tiled_list + nodes,
-        d->tiled_list + 2 * nodes);
+        d->cls, d->layout == LBX_LAYOUT_COMPACT ? d->fidx : nullptr, p.LX, p.LY, plan.K,
+        (Tile*)plan.tiles, plan.gidx, plan.list, plan.list + nodes, plan.list + 2 * nodes);
     d->launches++;
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {
-    lbx_internal_tiled_free(d);
-    d->tiled_state = -1;
-    if (e == cudaErrorMemoryAllocation && d->run_mode != LBX_RUN_TILED) {
-      cudaGetLastError();             // a launch per step needs none
+    if (e == cudaErrorMemoryAllocation && (l > 0 || d->run_mode != LBX_RUN_TILED)) {
+      cudaGetLastError();             // another level, or a launch per step
       return LBX_OK;
     }
     return lbx_internal_fail(e == cudaErrorMemoryAllocation ? LBX_ERR_NOMEM : LBX_ERR_CUDA,
                              cudaGetErrorString(e));
   }
-  d->tiled_state = 1;
+  plan.state = 1;
+  return LBX_OK;
+}
+
+lbx_status plan_level(lbx_domain* d, int l)
+{
+  if (d->tiled[l].state != 0) return LBX_OK;
+  try {
+    if (d->real_size == 8)
+      return d->p.nsubs == 2 ? make_plan<double, 2>(d, l) : make_plan<double, 1>(d, l);
+    return d->p.nsubs == 2 ? make_plan<float, 2>(d, l) : make_plan<float, 1>(d, l);
+  } catch (const std::bad_alloc&) {
+    d->tiled[l].state = -1;           // no host memory for it
+    return LBX_OK;
+  }
+}
+
+// ---- domains side by side ---------------------------------------------------
+
+// A tiled launch holds every SM that it has a block on.  With the GPU to
+// itself a domain's tiles spread over all SMs, where a small lattice spends
+// most of its time in halos and waits; launches of several domains, on
+// streams of their own, would then run one after another (twelve of 48 x 67,
+// 2000 steps each: FP64 26 ms, FP32 21; on a sixteenth of the GPU each, side
+// by side, 4.3 and 3.4; one alone 2.2 and 2.0).  So a launch looks whether
+// other domains' tiled runs are under way and takes tiles for its share.  The
+// results do not depend on the tiles: every node's update is the same code on
+// the same values.
+//
+// The listed domains are those that have launched a tiled run.  A launch
+// records its domain's event if another stream's domain is listed; one that
+// comes later asks whether the event has passed.  A domain that launched
+// after this one's last launch counts as busy if the newest of those still
+// is, which saves asking for each (a round of many domains would ask for all
+// the others in each launch).  A launch that others were seen beside leaves
+// their number for its domain's next one, which is the first of a new round
+// in a program that waits for all domains between rounds.
+std::mutex g_mu;                        // guards what follows, and the listed domains' fields
+std::vector<lbx_domain*> g_listed;      // tiled_stream, _turn, _busy and _company
+unsigned long long g_turn = 0;
+
+bool under_way(lbx_domain* o)
+{
+  if (!o->tiled_busy) return false;
+  const cudaError_t e = cudaEventQuery(o->tiled_done);
+  if (e != cudaErrorNotReady) o->tiled_busy = false;
+  if (e != cudaSuccess) cudaGetLastError();
+  return o->tiled_busy;
+}
+
+// Other domains' tiled runs under way on d's device; *beside: such domains
+// are listed at all.
+int busy_beside(lbx_domain* d, bool* beside)
+{
+  // a caller's capture elsewhere is none of these calls' business
+  struct Relaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  };
+  std::lock_guard<std::mutex> lock(g_mu);
+  if (!d->tiled_listed) try {
+    g_listed.push_back(d);
+    d->tiled_listed = true;
+  } catch (const std::bad_alloc&) {}    // unseen by the others
+  d->tiled_stream = d->stream;
+  lbx_domain* newest = nullptr;
+  *beside = false;
+  for (lbx_domain* o : g_listed) {
+    if (o == d || o->p.device != d->p.device || o->tiled_stream == d->stream) continue;
+    *beside = true;
+    if (o->tiled_busy && (!newest || o->tiled_turn > newest->tiled_turn)) newest = o;
+  }
+  const int company = d->tiled_company;
+  d->tiled_company = 0;
+  if (!newest) return company;
+  Relaxed relaxed;
+  const bool assume = under_way(newest);
+  auto counts = [&](const lbx_domain* o) {
+    return o != d && o->p.device == d->p.device && o->tiled_stream != d->stream && o->tiled_busy;
+  };
+  int n = 0;
+  for (lbx_domain* o : g_listed)
+    if (counts(o) && ((assume && o->tiled_turn > d->tiled_turn) || under_way(o))) ++n;
+  for (lbx_domain* o : g_listed)
+    if (counts(o)) o->tiled_company = std::max(o->tiled_company, n);
+  return std::max(n, company);
+}
+
+// After a launch: its event, if other domains are listed.
+void launched(lbx_domain* d, bool beside)
+{
+  bool busy = false;
+  if (beside) {
+    cudaError_t e = d->tiled_done ? cudaSuccess
+                                  : cudaEventCreateWithFlags(&d->tiled_done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(d->tiled_done, d->stream);
+    if (e != cudaSuccess) cudaGetLastError();
+    busy = e == cudaSuccess;
+  }
+  std::lock_guard<std::mutex> lock(g_mu);
+  d->tiled_turn = ++g_turn;
+  d->tiled_busy = busy;
+}
+
+template <typename T, int NS>
+void model_level(lbx_domain* d, int l)
+{
+  Shape shapes[kShapes];
+  if (d->tiled[l].us == 0.0) shapes_of<T, NS>(d, l, shapes);
+}
+
+// The level whose plan a launch beside n others takes: all of them are
+// modelled done soonest.
+lbx_status choose_level(lbx_domain* d, int n, int* level)
+{
+  *level = 0;
+  double best = d->tiled[0].us * (n + 1);
+  for (int l = 1; l < TiledPlan::kLevels && (1 << (l - 1)) < n + 1; ++l) {
+    if (d->real_size == 8) d->p.nsubs == 2 ? model_level<double, 2>(d, l) : model_level<double, 1>(d, l);
+    else d->p.nsubs == 2 ? model_level<float, 2>(d, l) : model_level<float, 1>(d, l);
+    const double us = d->tiled[l].us * ((n >> l) + 1);    // n + 1 runs, 2^l at a time
+    if (us >= best) continue;
+    if (lbx_status st = plan_level(d, l)) return st;
+    if (d->tiled[l].state <= 0) continue;
+    best = us;
+    *level = l;
+  }
   return LBX_OK;
 }
 
@@ -748,19 +911,23 @@ lbx_status launch(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
 {
   constexpr size_t smem = tiled_smem<T, NS>();
   const void* fn = (const void*)aa_tiled<T, NS, MODEL>;
-  const int nt = d->tiled_ntiles;
-  const int rounds = round_count(pairs, d->tiled_k);
   cudaError_t e = cudaSuccess;
   if (!d->tiled_attr) {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return lbx_internal_fail(LBX_ERR_CUDA, cudaGetErrorString(e));
     d->tiled_attr = true;
   }
-  if (d->tiled_base + rounds + 1 >= (1 << 30)) {
+  bool beside = false;
+  int level = 0;
+  if (const int n = busy_beside(d, &beside))
+    if (lbx_status st = choose_level(d, n, &level)) return st;
+  TiledPlan& plan = d->tiled[level];
+  const int rounds = round_count(pairs, plan.K);
+  if (plan.base + rounds + 1 >= (1 << 30)) {
     // restart the counters before they could wrap
-    e = cudaMemsetAsync(d->tiled_flags, 0, (size_t)nt * sizeof(int), d->stream);
+    e = cudaMemsetAsync(plan.flags, 0, (size_t)plan.ntiles * sizeof(int), d->stream);
     if (e != cudaSuccess) return lbx_internal_fail(LBX_ERR_CUDA, cudaGetErrorString(e));
-    d->tiled_base = 0;
+    plan.base = 0;
   }
   const bool compact = d->layout == LBX_LAYOUT_COMPACT;
   StepArgs<T> a = A;
@@ -768,24 +935,25 @@ lbx_status launch(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
   r.f0 = (T*)(compact ? d->fc : d->f);
   r.f1 = (T*)d->tiled_scratch;
   r.P = compact ? d->P : d->N;
-  r.tiles = (const Tile*)d->tiled_plan;
-  r.gidx = d->tiled_gidx;
-  r.list = d->tiled_list;
-  r.wrd = r.list + d->tiled_nodes;
-  r.halo = r.wrd + d->tiled_nodes;
-  r.nbrs = d->tiled_nbrs;
-  r.flags = d->tiled_flags;
-  r.status = d->tiled_flags + nt;
-  r.base = d->tiled_base;
-  r.K = d->tiled_k;
+  r.tiles = (const Tile*)plan.tiles;
+  r.gidx = plan.gidx;
+  r.list = plan.list;
+  r.wrd = r.list + plan.nodes;
+  r.halo = r.wrd + plan.nodes;
+  r.nbrs = plan.nbrs;
+  r.flags = plan.flags;
+  r.status = d->tiled_status;
+  r.base = plan.base;
+  r.K = plan.K;
   r.pairs = pairs;
   r.rounds = rounds;
   r.write_mv = write_mv ? 1 : 0;
   void* args[] = {&a, &r};
-  e = cudaLaunchCooperativeKernel(fn, nt, kTiledThreads, args, smem, d->stream);
+  e = cudaLaunchCooperativeKernel(fn, plan.ntiles, kTiledThreads, args, smem, d->stream);
   if (e != cudaSuccess) return lbx_internal_fail(LBX_ERR_CUDA, cudaGetErrorString(e));
-  d->tiled_base += rounds;
+  plan.base += rounds;
   d->launches++;
+  launched(d, beside);
   return LBX_OK;
 }
 
@@ -801,37 +969,24 @@ lbx_status run_ns(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
 
 size_t lbx_internal_tiled_room(lbx_domain* d)
 {
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d->p.device) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  if (d->fluid == 0 || d->host_solids.empty()) return 0;
-  if (d->real_size == 8) return d->p.nsubs == 2 ? room<double, 2>(d, sms) : room<double, 1>(d, sms);
-  return d->p.nsubs == 2 ? room<float, 2>(d, sms) : room<float, 1>(d, sms);
+  if (d->fluid == 0 || d->host_solids.empty() || multiprocessors(d) == 0) return 0;
+  if (d->real_size == 8) return d->p.nsubs == 2 ? room<double, 2>(d) : room<double, 1>(d);
+  return d->p.nsubs == 2 ? room<float, 2>(d) : room<float, 1>(d);
 }
 
 lbx_status lbx_internal_tiled_plan(lbx_domain* d, bool* yes)
 {
-  const lbx_params& p = d->p;
   *yes = false;
   if (d->host_solids.empty() || (d->run_mode != LBX_RUN_TILED && !better(d))) return LBX_OK;
-  if (d->tiled_state == 0) try {
-    lbx_status st = d->real_size == 8
-                        ? (p.nsubs == 2 ? make_plan<double, 2>(d) : make_plan<double, 1>(d))
-                        : (p.nsubs == 2 ? make_plan<float, 2>(d) : make_plan<float, 1>(d));
-    if (st != LBX_OK) return st;
-  } catch (const std::bad_alloc&) {
-    d->tiled_state = -1;              // no host memory for it either
-  }
-  *yes = d->tiled_state > 0;
+  if (lbx_status st = plan_level(d, 0)) return st;
+  *yes = d->tiled[0].state > 0;
   return LBX_OK;
 }
 
 template <typename T>
 lbx_status lbx_internal_tiled_run(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
 {
-  if (pairs < 2 || d->tiled_state <= 0)
+  if (pairs < 2 || d->tiled[0].state <= 0)
     return lbx_internal_fail(LBX_ERR_INVALID, "tiled run without a plan or two pairs");
   return d->p.nsubs == 2 ? run_ns<T, 2>(d, A, pairs, write_mv) : run_ns<T, 1>(d, A, pairs, write_mv);
 }
@@ -841,22 +996,34 @@ template lbx_status lbx_internal_tiled_run<double>(lbx_domain*, const StepArgs<d
 
 void lbx_internal_tiled_free(lbx_domain* d)
 {
-  if (d->tiled_own) { cudaFree(d->tiled_own); d->tiled_room = nullptr; }
-  d->tiled_own = d->tiled_plan = d->tiled_scratch = nullptr;
-  d->tiled_nbrs = d->tiled_gidx = d->tiled_flags = nullptr;
-  d->tiled_list = nullptr;
-  d->tiled_state = 0;
+  if (d->tiled_listed) {
+    std::lock_guard<std::mutex> lock(g_mu);
+    g_listed.erase(std::find(g_listed.begin(), g_listed.end(), d));
+    d->tiled_listed = false;
+  }
+  if (d->tiled_done) cudaEventDestroy(d->tiled_done);
+  d->tiled_done = nullptr;
+  for (TiledPlan& plan : d->tiled) {
+    cudaFree(plan.own);
+    plan = TiledPlan();
+  }
+  cudaFree(d->tiled_own);
+  d->tiled_own = d->tiled_scratch = d->tiled_tables = nullptr;
+  d->tiled_status = nullptr;
 }
 
 lbx_status lbx_internal_tiled_status(lbx_domain* d)
 {
-  if (!d->tiled_flags) return LBX_OK;
-  const int ntiles = d->tiled_ntiles;
+  if (!d->tiled_status) return LBX_OK;
   int st = 0;
-  cudaError_t e = cudaMemcpy(&st, d->tiled_flags + ntiles, sizeof(int), cudaMemcpyDeviceToHost);
+  cudaError_t e = cudaMemcpy(&st, d->tiled_status, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return lbx_internal_fail(LBX_ERR_CUDA, cudaGetErrorString(e));
   if (st == 0) return LBX_OK;
-  cudaMemset(d->tiled_flags, 0, (size_t)(ntiles + 1) * sizeof(int));
-  d->tiled_base = 0;
+  cudaMemset(d->tiled_status, 0, sizeof(int));
+  for (TiledPlan& plan : d->tiled) {
+    if (plan.state <= 0) continue;
+    cudaMemset(plan.flags, 0, (size_t)plan.ntiles * sizeof(int));
+    plan.base = 0;
+  }
   return lbx_internal_fail(LBX_ERR_CUDA, "tiled run: a block's wait for its neighbours ran out");
 }
