@@ -594,12 +594,10 @@ aa_step(StepArgs<T> A, FastDiv div_plane, FastDiv div_lx)
   __shared__ Idx sslot[ODD ? Q : 1][256];
   // Node indices are 32-bit (the host rejects N >= 2^31).
   const unsigned nu = blockIdx.x * 256u + threadIdx.x;
+  if (nu >= (unsigned)A.N) return;
   const int n = (int)nu;
-  const uint8_t cl = WALSH || nu >= (unsigned)A.N ? uint8_t(0) : A.cls[n];
-  // whether a node of the warp is next to a solid, while all its lanes are here
-  const bool near = ODD && !WALSH &&
-                    __any_sync(0xffffffffu, (cl & (CLS_NEAR | CLS_SOLID)) == CLS_NEAR);
-  if (nu >= (unsigned)A.N || (cl & CLS_SOLID)) return;
+  const uint8_t cl = WALSH ? uint8_t(0) : A.cls[n];
+  if (cl & CLS_SOLID) return;
   pdl_wait();
   const Idx N = (Idx)A.N;
 
@@ -649,7 +647,7 @@ aa_step(StepArgs<T> A, FastDiv div_plane, FastDiv div_lx)
                + (cz(a) < 0 ? zm : (cz(a) > 0 ? zp : 0));
         };
         // a warp with no node next to a solid forms no selects
-        if (near) {
+        if (!WALSH && __any_sync(__activemask(), cl & CLS_NEAR)) {
           const uint32_t nb = (cl & CLS_NEAR) ? A.nbm[n] : 0u;
 #pragma unroll
           for (int a = 0; a < Q; ++a)
