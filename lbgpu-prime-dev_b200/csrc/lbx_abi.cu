@@ -294,10 +294,12 @@ void launch_nodes(lbx_domain* d, const StepArgs<T>& A, bool odd, const Face3Fuse
   const bool idx32 = (unsigned long long)Q * (unsigned long long)A.N < (1ull << 32);
   auto go = [&](auto odd_c, auto idx_c, auto walsh_c) {
     constexpr bool o = decltype(odd_c)::value;
-    if constexpr (step_joint<Q, NS, o, false>() == (PART == PART_ALL))
-      launch_step_kernel(aa_step<T, Q, NS, MODEL, o, PART, decltype(idx_c)::value,
-                                 decltype(walsh_c)::value>,
-                         (unsigned)((A.N + 255) / 256), 256, d->stream, dependent, A, dp, dl);
+    constexpr bool w = decltype(walsh_c)::value;
+    if constexpr (step_joint<Q, NS, o, false>() == (PART == PART_ALL)) {
+      const unsigned bs = dense_block<T, Q, NS, w>(A.N);
+      launch_step_kernel(aa_step<T, Q, NS, MODEL, o, PART, decltype(idx_c)::value, w>,
+                         (unsigned)((A.N + bs - 1) / bs), bs, d->stream, dependent, A, dp, dl);
+    }
   };
   if (A.ns) {
     if (idx32) { if (odd) go(TT{}, TT{}, TT{}); else go(FF{}, TT{}, TT{}); }

@@ -559,19 +559,43 @@ __device__ __forceinline__ void face_south(int kind, T rho_bc, T rhoA, T drho, b
 template <bool CG, typename T>
 __device__ __forceinline__ T ld_pop(const T* p) { return CG ? __ldcg(p) : *p; }
 
-// Resident 256-thread blocks of the dense kernels: FP32 six (40 registers;
-// four with two substances in one thread, five for a solute launch), FP64
-// three (80; four for D2Q9's 64, two with two substances or for a solute
-// launch); Walsh kernels hold the incoming populations too.  Measured at 193 x 161 x 120: FP32 odd 105 us at six or five, 109 at
-// four or seven; even 94 us at six, 101 at four; FP64 odd 185 us at three,
-// 221 at two.
+// Threads per block (at most: see dense_block) and resident blocks of the
+// dense kernels.  FP32: 256, six (40 registers; four with two substances in
+// one thread, five for a solute launch); at 193 x 161 x 120 odd 105 us at six
+// or five, 109 at four or seven, even 94 at six, 101 at four.  FP64: 128, six
+// for D3Q19 (80 registers; odd 185 us, 221 at 128), five for a solute launch
+// (96; at 80 the odd one spills), eight for D2Q9 (64), four with two
+// substances in one thread; Walsh kernels hold the incoming populations too,
+// D3Q19 five.  With 256-thread blocks, two or three of them, FP64 steps left
+// registers idle (us per step, 256 then 128 threads): D2Q9 1000 x 1100 20.7,
+// 19.5, with Walsh nodes 26.7, 22.5; 128^3 with a solute 262, 254; 97 x 83 x
+// 61 with Walsh nodes 24.0, 20.2.
+template <typename T>
+__host__ __device__ constexpr int dense_threads() { return sizeof(T) == 8 ? 128 : 256; }
+
 template <typename T, int Q, int NS, int PART, bool WALSH>
 __host__ __device__ constexpr int dense_min_blocks()
 {
-  return (PART == PART_ALL && NS == 2) ? (sizeof(T) == 4 && !WALSH ? 4 : 2)
-       : PART == PART_SOLUTE           ? (sizeof(T) == 4 ? (WALSH ? 3 : 5) : 2)
-       : sizeof(T) == 4                ? (WALSH ? 4 : 6)
-                                       : (WALSH ? 2 : (Q == 9 ? 4 : 3));
+  if (sizeof(T) == 8)
+    return (PART == PART_ALL && NS == 2) ? 4
+         : Q == 9                        ? 8
+                                         : (WALSH || PART == PART_SOLUTE ? 5 : 6);
+  return (PART == PART_ALL && NS == 2) ? (WALSH ? 2 : 4)
+       : PART == PART_SOLUTE           ? (WALSH ? 3 : 5)
+                                       : (WALSH ? 4 : 6);
+}
+
+// The threads per block of a launch over `nodes` nodes: fewer where 256 leave
+// SMs without a block (24 x 20 x 18 FP32 with z faces 5.47 us per step, 64
+// threads 5.16, FP64 with a solute 10.1, 8.9; 64 x 48 FP32 2.02, 128 threads
+// 1.81), and 128 for the FP32 D2Q9 kernels of many registers (2000 x 1500
+// with a solute 92.3, 87.8, with Walsh nodes 45.6, 43.9); the other FP32 ones
+// stream faster with 256 (80^3 11.9 against 12.6).
+template <typename T, int Q, int NS, bool WALSH>
+constexpr unsigned dense_block(long long nodes)
+{
+  if (nodes < 16384) return Q == 9 ? 128 : 64;
+  return Q == 9 && (WALSH || NS == 2) ? 128 : dense_threads<T>();
 }
 
 // One thread per node, the nodes numbered through (no block starts anew at
@@ -586,14 +610,14 @@ __host__ __device__ constexpr int dense_min_blocks()
 // 231 -> 185 us FP64).  IDX32: offsets within one substance's [Q][N] block
 // fit in 32 bits.
 template <typename T, int Q, int NS, int MODEL, bool ODD, int PART, bool IDX32, bool WALSH = false>
-__global__ void __launch_bounds__(256, (dense_min_blocks<T, Q, NS, PART, WALSH>()))
+__global__ void __launch_bounds__(dense_threads<T>(), (dense_min_blocks<T, Q, NS, PART, WALSH>()))
 aa_step(StepArgs<T> A, FastDiv div_plane, FastDiv div_lx)
 {
   using Idx = typename std::conditional<IDX32, unsigned, size_t>::type;
   constexpr int D = (Q == 9) ? 2 : 3;
-  __shared__ Idx sslot[ODD ? Q : 1][256];
+  __shared__ Idx sslot[ODD ? Q : 1][dense_threads<T>()];
   // Node indices are 32-bit (the host rejects N >= 2^31).
-  const unsigned nu = blockIdx.x * 256u + threadIdx.x;
+  const unsigned nu = blockIdx.x * blockDim.x + threadIdx.x;
   if (nu >= (unsigned)A.N) return;
   const int n = (int)nu;
   const uint8_t cl = WALSH ? uint8_t(0) : A.cls[n];
@@ -646,7 +670,9 @@ aa_step(StepArgs<T> A, FastDiv div_plane, FastDiv div_lx)
           return (cx(a) < 0 ? xm : (cx(a) > 0 ? xp : 0)) + (cy(a) < 0 ? ym : (cy(a) > 0 ? yp : 0))
                + (cz(a) < 0 ? zm : (cz(a) > 0 ? zp : 0));
         };
-        // a warp with no node next to a solid forms no selects
+        // a warp with no node next to a solid forms no selects (every lane that
+        // reads a mask goes on to the vote with it; any mask gives its lanes a
+        // right answer)
         if (!WALSH && __any_sync(__activemask(), cl & CLS_NEAR)) {
           const uint32_t nb = (cl & CLS_NEAR) ? A.nbm[n] : 0u;
 #pragma unroll
