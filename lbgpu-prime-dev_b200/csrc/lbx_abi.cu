@@ -1214,11 +1214,13 @@ lbx_status lbx_run(lbx_domain* d, int t0, int nsteps, int frame_rate)
         if (lbx_status st = tiled_applies(d, t, &tiled)) return st;
       if (tiled) {
         if (lbx_status st = tiled_pairs(d, t, all, frame_last)) return st;
+        lbx_internal_tiled_launched(d);
         t += 2 * all;
         continue;
       }
       if (pairs >= 2) {
         if (lbx_status st = replay_pairs(d, t, pairs)) return st;
+        lbx_internal_tiled_launched(d);
         t += 2 * pairs;
         continue;
       }

@@ -99,6 +99,8 @@ struct lbx_domain {
   void* tiled_scratch = nullptr;         // a second population array for its rounds
   int* tiled_status = nullptr;           // set by a launch whose wait ran out
   void* tiled_tables = nullptr;          // room for the first plan's tables
+  int tiled_level = 0;                   // the plan of the next launch, -1: a launch per step
+  bool tiled_beside = false;             // other streams' domains are listed
   // its last launch, for other domains' (guarded by the mutex in lbx_tiled.cu,
   // but for the event itself)
   cudaEvent_t tiled_done = nullptr;
@@ -141,9 +143,11 @@ LBX_HIDDEN lbx_status lbx_internal_pest_after(lbx_domain* d, int t);
 LBX_HIDDEN void lbx_internal_pest_free(lbx_domain* d);
 // Temporal blocking.  At creation: bytes the tiled run of this lattice would
 // like behind the population array (0: it would not be taken).  Then whether
-// the domain's run mode takes it, the tiles planned on first use; then
-// `pairs` AA pairs (two or more) with the launch arguments A from the state
-// after an even step, the last step writing the macro variables if asked.
+// the domain's run mode takes it for the stretch to be launched, the tiles
+// planned on first use; then `pairs` AA pairs (two or more) with the launch
+// arguments A from the state after an even step, the last step writing the
+// macro variables if asked; and after the stretch's launches, tiled or not,
+// tiled_launched.
 LBX_HIDDEN size_t lbx_internal_tiled_room(lbx_domain* d);
 // Whether the caller is capturing `stream` into a graph of its own.
 LBX_HIDDEN bool lbx_internal_capturing(cudaStream_t stream);
@@ -151,6 +155,7 @@ LBX_HIDDEN lbx_status lbx_internal_tiled_plan(lbx_domain* d, bool* yes);
 template <typename T>
 LBX_HIDDEN lbx_status lbx_internal_tiled_run(lbx_domain* d, const lbx::StepArgs<T>& A, int pairs,
                                              bool write_mv);
+LBX_HIDDEN void lbx_internal_tiled_launched(lbx_domain* d);
 LBX_HIDDEN void lbx_internal_tiled_free(lbx_domain* d);
 // LBX_OK, or the error of a tiled launch whose bounded wait ran out (then
 // cleared); synchronous.

@@ -804,8 +804,8 @@ lbx_status plan_level(lbx_domain* d, int l)
 // results do not depend on the tiles: every node's update is the same code on
 // the same values.
 //
-// The listed domains are those that have launched a tiled run.  A launch
-// records its domain's event if another stream's domain is listed; one that
+// The listed domains are those that have taken, or might have taken, a tiled
+// run.  A stretch's launch records its domain's event if another stream's domain is listed; one that
 // comes later asks whether the event has passed.  A domain that launched
 // after this one's last launch counts as busy if the newest of those still
 // is, which saves asking for each (a round of many domains would ask for all
@@ -864,11 +864,14 @@ int busy_beside(lbx_domain* d, bool* beside)
   return std::max(n, company);
 }
 
-// After a launch: its event, if other domains are listed.
-void launched(lbx_domain* d, bool beside)
+}  // namespace
+
+// After the stretch's launches: the domain's event, if others are listed.
+void lbx_internal_tiled_launched(lbx_domain* d)
 {
+  if (!d->tiled_listed) return;
   bool busy = false;
-  if (beside) {
+  if (d->tiled_beside) {
     cudaError_t e = d->tiled_done ? cudaSuccess
                                   : cudaEventCreateWithFlags(&d->tiled_done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventRecord(d->tiled_done, d->stream);
@@ -880,6 +883,8 @@ void launched(lbx_domain* d, bool beside)
   d->tiled_busy = busy;
 }
 
+namespace {
+
 template <typename T, int NS>
 void model_level(lbx_domain* d, int l)
 {
@@ -887,8 +892,12 @@ void model_level(lbx_domain* d, int l)
   if (d->tiled[l].us == 0.0) shapes_of<T, NS>(d, l, shapes);
 }
 
-// The level whose plan a launch beside n others takes: all of them are
-// modelled done soonest.
+// The level whose plan a launch beside n others takes, with which all of them
+// are modelled done soonest, and that time per step; -1: a launch per step.
+// Step launches run beside one another without holding SMs, so they win
+// where the lattice is large for a share of the GPU (three 300 x 300 FP64,
+// 800 steps: tiled 4.9 ms, step launches 3.8).  FP32 does not take them here:
+// its results would depend on the others in their last bits.
 lbx_status choose_level(lbx_domain* d, int n, int* level)
 {
   *level = 0;
@@ -903,6 +912,10 @@ lbx_status choose_level(lbx_domain* d, int n, int* level)
     best = us;
     *level = l;
   }
+  // (its launches cost the host more: by some margin)
+  if (n > 0 && d->real_size == 8 && d->run_mode == LBX_RUN_AUTO &&
+      1.15 * steps_us((double)d->fluid * (n + 1), d->real_size, d->p.nsubs) < best)
+    *level = -1;
   return LBX_OK;
 }
 
@@ -917,11 +930,7 @@ lbx_status launch(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
     if (e != cudaSuccess) return lbx_internal_fail(LBX_ERR_CUDA, cudaGetErrorString(e));
     d->tiled_attr = true;
   }
-  bool beside = false;
-  int level = 0;
-  if (const int n = busy_beside(d, &beside))
-    if (lbx_status st = choose_level(d, n, &level)) return st;
-  TiledPlan& plan = d->tiled[level];
+  TiledPlan& plan = d->tiled[d->tiled_level];
   const int rounds = round_count(pairs, plan.K);
   if (plan.base + rounds + 1 >= (1 << 30)) {
     // restart the counters before they could wrap
@@ -953,7 +962,6 @@ lbx_status launch(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
   if (e != cudaSuccess) return lbx_internal_fail(LBX_ERR_CUDA, cudaGetErrorString(e));
   plan.base += rounds;
   d->launches++;
-  launched(d, beside);
   return LBX_OK;
 }
 
@@ -979,14 +987,17 @@ lbx_status lbx_internal_tiled_plan(lbx_domain* d, bool* yes)
   *yes = false;
   if (d->host_solids.empty() || (d->run_mode != LBX_RUN_TILED && !better(d))) return LBX_OK;
   if (lbx_status st = plan_level(d, 0)) return st;
-  *yes = d->tiled[0].state > 0;
+  if (d->tiled[0].state <= 0) return LBX_OK;
+  const int n = busy_beside(d, &d->tiled_beside);
+  if (lbx_status st = choose_level(d, n, &d->tiled_level)) return st;
+  *yes = d->tiled_level >= 0;
   return LBX_OK;
 }
 
 template <typename T>
 lbx_status lbx_internal_tiled_run(lbx_domain* d, const StepArgs<T>& A, int pairs, bool write_mv)
 {
-  if (pairs < 2 || d->tiled[0].state <= 0)
+  if (pairs < 2 || d->tiled_level < 0 || d->tiled[d->tiled_level].state <= 0)
     return lbx_internal_fail(LBX_ERR_INVALID, "tiled run without a plan or two pairs");
   return d->p.nsubs == 2 ? run_ns<T, 2>(d, A, pairs, write_mv) : run_ns<T, 1>(d, A, pairs, write_mv);
 }

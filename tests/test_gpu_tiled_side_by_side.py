@@ -33,7 +33,8 @@ def _state(d):
 @pytest.mark.parametrize("threads", [False, True])
 @pytest.mark.parametrize("real,nsubs", [(8, 1), (4, 1), (8, 2)])
 def test_results_do_not_depend_on_the_others(real, nsubs, threads):
-    shapes = [(48, 67), (30, 30), (100, 64), (128, 128), (17, 41), (64, 64), (200, 90)]
+    shapes = [(48, 67), (30, 30), (100, 64), (128, 128), (17, 41), (64, 64), (200, 90), (300, 300),
+              (256, 256)]
     calls = [(40, 40), (20, 60), (200, 0), (6, 266), (34, 300)]
 
     def go(d):
