@@ -148,13 +148,16 @@ __device__ __forceinline__ void batch_block(const BatchArgs<T>& A, int b)
   batch_node<T, Q, MODEL, ODD, IDX32>(A.blkdesc[b], A, b * blockDim.x + threadIdx.x);
 }
 
-template <typename T, bool ODD>
-constexpr int batch_min_blocks() { return sizeof(T) == 4 ? (ODD ? 6 : 4) : 3; }
+// Up to 256 threads per block.  Resident blocks: FP32 six (40 registers), the
+// even step too, unlike a single lattice's: a block's position table and
+// descriptor are two more loads in a chain, which more warps hide (256
+// samples of edges 32 to 96, a step 1.198 ms; with the even step at four
+// blocks 1.232, at five 1.205); FP64 three.
+template <typename T>
+constexpr int batch_min_blocks() { return sizeof(T) == 4 ? 6 : 3; }
 
-// Up to 256 threads per block, resident blocks as for the single-lattice
-// compact kernels (FP64 three).
 template <typename T, int Q, int MODEL, bool ODD, bool IDX32>
-__global__ void __launch_bounds__(256, (batch_min_blocks<T, ODD>()))
+__global__ void __launch_bounds__(256, (batch_min_blocks<T>()))
 aa_step_batch(BatchArgs<T> A)
 {
   batch_block<T, Q, MODEL, ODD, IDX32>(A, A.block0 + blockIdx.x);
@@ -165,7 +168,7 @@ aa_step_batch(BatchArgs<T> A)
 // in the pool instead cost the odd step 3-6 %: nine dependent constant-cache
 // reads that miss when 512 samples' tables share an SM's constant cache.)
 template <typename T, int Q, int MODEL, bool ODD, bool IDX32>
-__global__ void __launch_bounds__(256, (batch_min_blocks<T, ODD>()))
+__global__ void __launch_bounds__(256, (batch_min_blocks<T>()))
 aa_step_batch_pool(BatchArgs<T> A, PoolRef R)
 {
   const int bl = R.block0 + blockIdx.x;
