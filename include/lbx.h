@@ -218,6 +218,9 @@ lbx_status lbx_set_stream(lbx_domain* d, void* stream);
  *                  cooperative launch runs rounds of up to 12 steps on tiles
  *                  held in shared memory with halos as deep; FP64 results
  *                  are bit-identical to STEPS.
+ * Domains whose tiled runs are under way side by side (streams of their own,
+ * one device) take tiles for a share of the GPU each, with the same results;
+ * in FP64 AUTO then also takes STEPS where that is the faster one.
  * LBX_ERR_INVALID for another mode. */
 enum { LBX_RUN_AUTO = 0, LBX_RUN_STEPS = 1, LBX_RUN_TILED = 2 };
 lbx_status lbx_set_run_mode(lbx_domain* d, int mode);

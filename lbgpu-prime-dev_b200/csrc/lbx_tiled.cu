@@ -37,7 +37,8 @@
 // about equal work per round (fluid node updates, halo included): the
 // slowest tile sets the pace, and the fluid fraction of fixed tiles of a
 // porous lattice spreads from below 0.3 to near 1.  Width, rows per column
-// and K come from a small cost model (see best_shapes).  The tiles' node
+// and K come from a small cost model (see best_shapes), for all SMs or, beside
+// other domains' runs, for a share of them (choose_level).  The tiles' node
 // tables are made once, on the device (tile_tables), and read by every
 // launch: made anew in each launch they cost 15-20 us, more than the 20
 // steps between two frames of a small lattice.
@@ -805,13 +806,14 @@ lbx_status plan_level(lbx_domain* d, int l)
 // the same values.
 //
 // The listed domains are those that have taken, or might have taken, a tiled
-// run.  A stretch's launch records its domain's event if another stream's domain is listed; one that
-// comes later asks whether the event has passed.  A domain that launched
-// after this one's last launch counts as busy if the newest of those still
-// is, which saves asking for each (a round of many domains would ask for all
-// the others in each launch).  A launch that others were seen beside leaves
-// their number for its domain's next one, which is the first of a new round
-// in a program that waits for all domains between rounds.
+// run.  A stretch's launch records its domain's event if another stream's
+// domain is listed; one that comes later asks whether the event has passed.
+// A domain that launched after this one's last launch counts as busy if the
+// newest of those still is, which saves asking for each (a round of many
+// domains would ask for all the others in each launch).  A launch that others
+// were seen beside leaves their number for its domain's next one, which is
+// the first of a new round in a program that waits for all domains between
+// rounds.
 std::mutex g_mu;                        // guards what follows, and the listed domains' fields
 std::vector<lbx_domain*> g_listed;      // tiled_stream, _turn, _busy and _company
 unsigned long long g_turn = 0;
@@ -893,7 +895,7 @@ void model_level(lbx_domain* d, int l)
 }
 
 // The level whose plan a launch beside n others takes, with which all of them
-// are modelled done soonest, and that time per step; -1: a launch per step.
+// are modelled done soonest; -1: a launch per step.
 // Step launches run beside one another without holding SMs, so they win
 // where the lattice is large for a share of the GPU (three 300 x 300 FP64,
 // 800 steps: tiled 4.9 ms, step launches 3.8).  FP32 does not take them here:
@@ -903,8 +905,10 @@ lbx_status choose_level(lbx_domain* d, int n, int* level)
   *level = 0;
   double best = d->tiled[0].us * (n + 1);
   for (int l = 1; l < TiledPlan::kLevels && (1 << (l - 1)) < n + 1; ++l) {
-    if (d->real_size == 8) d->p.nsubs == 2 ? model_level<double, 2>(d, l) : model_level<double, 1>(d, l);
-    else d->p.nsubs == 2 ? model_level<float, 2>(d, l) : model_level<float, 1>(d, l);
+    if (d->real_size == 8)
+      d->p.nsubs == 2 ? model_level<double, 2>(d, l) : model_level<double, 1>(d, l);
+    else
+      d->p.nsubs == 2 ? model_level<float, 2>(d, l) : model_level<float, 1>(d, l);
     const double us = d->tiled[l].us * ((n >> l) + 1);    // n + 1 runs, 2^l at a time
     if (us >= best) continue;
     if (lbx_status st = plan_level(d, l)) return st;
