@@ -100,7 +100,7 @@ struct lbx_domain {
   int* tiled_status = nullptr;           // set by a launch whose wait ran out
   void* tiled_tables = nullptr;          // room for the first plan's tables
   int tiled_level = 0;                   // the plan of the next launch, -1: a launch per step
-  bool tiled_beside = false;             // other streams' domains are listed
+  bool tiled_record = false;             // the stretch's launches are to be seen by other domains'
   // its last launch, for other domains' (guarded by the mutex in lbx_tiled.cu,
   // but for the event itself)
   cudaEvent_t tiled_done = nullptr;
