@@ -219,10 +219,9 @@ cudaError_t lbx_internal_copy_planes_out(int device, cudaStream_t stream, void* 
 {
   for (int c = 0, n = 1; c < count; c += n, n = 1) {
     if (!dst[c]) continue;
-    if (count * plane >= kStaged)
-      while (c + n < count && dst[c + n] == (char*)dst[c] + n * plane && pageable(dst[c]) &&
-             pageable(dst[c + n]))
-        ++n;
+    while (c + n < count && dst[c + n] == (char*)dst[c] + n * plane && pageable(dst[c]) &&
+           pageable(dst[c + n]))
+      ++n;
     const cudaError_t e =
         copy(device, stream, dst[c], (const char*)src + c * plane, n * plane, true);
     if (e != cudaSuccess) return e;

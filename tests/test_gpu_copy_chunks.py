@@ -32,7 +32,12 @@ def test_one_domain_per_job_does_not_pay_for_chunks():
             d.init_equilibrium(0, src)
         return time.perf_counter() - at
 
-    took = {k: sorted(job(v) for _ in range(7))[3] for k, v in rho.items()}
+    # the least of several in turn: page work of the host's other programs can
+    # take tens of milliseconds of any one
+    took = dict.fromkeys(rho, 1.0)
+    for _ in range(12):
+        for k, v in rho.items():
+            took[k] = min(took[k], job(v))
     assert took["pageable"] < took["locked"] + 6e-3, took
 
 

@@ -17,7 +17,7 @@ def _pages(count):
 
 
 @pytest.mark.parametrize("locked", [(), (0,), (1,), (0, 2), (0, 1, 2, 3), (3,)])
-@pytest.mark.parametrize("n", [4096 * 64, 4096 * 640])
+@pytest.mark.parametrize("n", [4096, 4096 * 64, 4096 * 640])
 def test_some_planes_page_locked(locked, n):
     import torch
     from lbx.batch import Batch
