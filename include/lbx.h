@@ -188,9 +188,9 @@ lbx_status lbx_step_pair(lbx_domain* d, int time, unsigned flags);
  * frame-free steps with unchanged launch arguments are replayed from CUDA
  * graphs (one AA pair, or eight pairs per graph launch; captured on first
  * use and kept while the arguments and the stream stay the same) but for
- * short stretches of large lattices, whose steps are launched directly until
- * 64 pairs with the same arguments have run.  In a stream that the caller is
- * capturing every step is a launch of its own.
+ * short stretches of large lattices, whose steps are launched directly (with
+ * z faces or a record until 64 pairs with the same arguments have run).  In a
+ * stream that the caller is capturing every step is a launch of its own.
  * Asynchronous. */
 lbx_status lbx_run(lbx_domain* d, int t0, int nsteps, int frame_rate);
 

@@ -802,9 +802,12 @@ lbx_status capture_pairs(lbx_domain* d, int t, int npairs, cudaGraphExec_t* out,
 // of the GPU, and capturing the graphs would hold it up (1-2 ms for a step
 // with z faces and a record, the GPU time of 30 such steps at 128 x 112 x
 // 96).  Populations of 50 MB (100 moved) step in some 20 us, more than the
-// launches of a step with faces take.  Stretches that add up to more pairs
-// with the same arguments throughout have earned the capture: it is the
-// program's loop.
+// launches of a step with faces take, if not by much: where a step is several
+// launches and event calls (z faces, a record), stretches that add up to more
+// pairs with the same arguments throughout have earned the capture.  Where it
+// is one launch or two they stay direct: dependent launches follow one another
+// more closely than graphs do (51 x 336 x 113 FP32, 11 pairs: 811 us, replayed
+// 820).
 constexpr int kGraphPairs = 8;
 constexpr int kDirectPairs = 64;
 constexpr double kDirectBytes = 50e6;
@@ -822,7 +825,7 @@ lbx_status replay_pairs(lbx_domain* d, int t, int pairs)
                          (double)(d->layout == LBX_LAYOUT_COMPACT ? d->fluid : d->N);
     const bool again = d->direct_stream == d->stream && d->direct_key_len == klen &&
                        std::memcmp(d->direct_key, key, klen) == 0;
-    d->direct_pairs = (again ? d->direct_pairs : 0) + pairs;
+    d->direct_pairs = (again && (d->faces3_active || d->btc_vals) ? d->direct_pairs : 0) + pairs;
     if (d->direct_pairs < kDirectPairs && bytes > kDirectBytes) {
       std::memcpy(d->direct_key, key, klen);
       d->direct_key_len = klen;
